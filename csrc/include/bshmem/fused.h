@@ -79,6 +79,11 @@ typedef struct {
 
 /* Launches the kernel on `stream`.  Returns a BSHMEM_FUSED_* code. */
 int bshmem_fused_gemm(const bshmem_fused_args_t* args, cudaStream_t stream);
+/* The same with operands stored transposed: `layout` is a sum of BSHMEM_FUSED_A_TRANSPOSED (A is [K][M], row-major; one PE
+ * only) and BSHMEM_FUSED_B_TRANSPOSED (B is [K][N]).  Not for GROUPED. */
+#define BSHMEM_FUSED_A_TRANSPOSED 1
+#define BSHMEM_FUSED_B_TRANSPOSED 2
+int bshmem_fused_gemm_layout(const bshmem_fused_args_t* args, int layout, cudaStream_t stream);
 int bshmem_fused_gemm_smem_bytes(void);
 
 #ifdef __cplusplus

@@ -151,6 +151,19 @@ __device__ __forceinline__ uint64_t umma_desc_k_sw128(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;           // SWIZZLE_128B
   return d;
 }
+// Shared-memory operand, MN-major, 128-byte swizzle: a tile is a row of blocks of 64 M/N elements; inside a block every
+// k has 128 bytes (its 64 elements), groups of 8 k are 1024 bytes apart (stride byte offset) and the next 64 M/N
+// elements are `block_bytes` away (leading byte offset).  16 values of k are 2048 bytes = 128 address units.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t block_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3ffff) >> 4);
+  d |= (uint64_t)(block_bytes >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+constexpr uint32_t UMMA_A_MN_MAJOR = 1u << 15, UMMA_B_MN_MAJOR = 1u << 16;  // instruction descriptor: transposed operands
 // Instruction descriptor, kind::f16: D fp32, A and B bf16, both K-major, no negation.
 // Bits: [4,6) D format (1 = f32), [7,10) A format (1 = bf16), [10,13) B format,
 // 15/16 A/B major (0 = K), [17,23) N>>3, [24,29) M>>4.

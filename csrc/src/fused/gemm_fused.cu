@@ -1,7 +1,9 @@
 // Fused tensor-parallel GEMM + collective for sm_100a, hand-written on
 // tcgen05 / tensor memory / TMA.
 //
-//   C[M,N] = A[M,K] · B[N,K]^T      A, B, C bf16 (both operands K-major), fp32 accumulation in TMEM
+//   C[M,N] = A[M,K] · B[N,K]^T      A, B, C bf16, fp32 accumulation in TMEM
+// Both operands are K-major by default; either may instead be stored with K outermost ([K][M], [K][N]), as the operands of
+// a linear layer's gradients are: the loads then take boxes of 64 contiguous rows x 64 k and the MMA reads them MN-major.
 //
 // One persistent CTA per SM, 256 threads, warp-specialised:
 //   warp 0    TMA producer   4-stage ring of {A 128x64, B 256x64} tiles (128-byte swizzle)
@@ -54,11 +56,14 @@ using namespace sm100;
 // CTA's tensor memory receives its own 128 x 256 accumulator: per SM, half the B traffic from L2 and
 // half the shared-memory reads per FLOP.  Everything after the accumulator (epilogue, flags, stores)
 // is per CTA and identical in both variants.
-template <bool PAIR>
+// MN = true: an operand may be stored with K outermost (p.a_mn, p.b_mn); compiled apart because the tests inside the loops of
+// the loading and the issuing thread cost the K-major case 1 us of 17 at 1152 x 2816 x 1984.
+template <bool PAIR, bool MN>
 __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_constant__ FusedParams p) {
   constexpr int STAGES = PAIR ? 6 : 4;
   constexpr int B_ROWS = PAIR ? BN / 2 : BN;
   constexpr int B_STAGE = B_ROWS * BK * 2;
+  constexpr int MN_BLOCK = 64 * BK * 2;  // MN-major operands: bytes of one block of 64 rows x 64 k
   static_assert(STAGES * (A_STAGE + B_STAGE) + EPI_BUFS * EPI_BUF == SMEM_TILES, "both variants use the same shared-memory budget");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -141,15 +146,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
         }
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, p.wait_limit_ns, abort_flag)) break;
-          if (PAIR) {
-            const uint32_t lead = mapa_u32(smem_u32(&full[stage]), 0);
-            mbar_expect_tx_cluster(lead, A_STAGE + B_STAGE);
-            tma_load_2d_pair(sA + stage * A_STAGE, &p.tmA, lead, kb * BK, ti.a_row);
-            tma_load_2d_pair(sB + stage * B_STAGE, &p.tmB, lead, kb * BK, ti.b_row + (int)cta_rank * B_ROWS);
+          const uint32_t lead = PAIR ? mapa_u32(smem_u32(&full[stage]), 0) : 0;
+          if (PAIR) mbar_expect_tx_cluster(lead, A_STAGE + B_STAGE);
+          else mbar_expect_tx(&full[stage], A_STAGE + B_STAGE);
+          auto load = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
+            if (PAIR) tma_load_2d_pair(dst, map, lead, x, y);
+            else tma_load_2d(dst, map, &full[stage], x, y);
+          };
+          // K-major operand: one box of 64 k x all rows.  MN-major operand: boxes of 64 rows (contiguous) x 64 k.
+          if (MN && p.a_mn) {
+#pragma unroll
+            for (int i = 0; i < BM / 64; ++i) load(sA + stage * A_STAGE + i * MN_BLOCK, &p.tmA, ti.a_row + i * 64, kb * BK);
           } else {
-            mbar_expect_tx(&full[stage], A_STAGE + B_STAGE);
-            tma_load_2d(sA + stage * A_STAGE, &p.tmA, &full[stage], kb * BK, ti.a_row);
-            tma_load_2d(sB + stage * B_STAGE, &p.tmB, &full[stage], kb * BK, ti.b_row);
+            load(sA + stage * A_STAGE, &p.tmA, kb * BK, ti.a_row);
+          }
+          const int b_row = ti.b_row + (PAIR ? (int)cta_rank * B_ROWS : 0);
+          if (MN && p.b_mn) {
+#pragma unroll
+            for (int i = 0; i < B_ROWS / 64; ++i) load(sB + stage * B_STAGE + i * MN_BLOCK, &p.tmB, b_row + i * 64, kb * BK);
+          } else {
+            load(sB + stage * B_STAGE, &p.tmB, kb * BK, b_row);
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -164,7 +180,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
   } else if (warp == 1) {
     // ---------------- MMA issuer
     if ((!PAIR || cta_rank == 0) && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16_f32(PAIR ? 2 * BM : BM, BN);
+      const uint32_t idesc = umma_idesc_bf16_f32(PAIR ? 2 * BM : BM, BN) | (MN && p.a_mn ? UMMA_A_MN_MAJOR : 0u) | (MN && p.b_mn ? UMMA_B_MN_MAJOR : 0u);
+      // Per 16 values of k: +32 bytes inside the 128-byte swizzle atom of a K-major operand (2 address units), two
+      // groups of 8 k (2048 bytes, 128 units) in an MN-major one.
+      const uint64_t a_step = MN && p.a_mn ? 128 : 2, b_step = MN && p.b_mn ? 128 : 2;
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       for (int t = first; t < total_tiles && !*abort_flag; t += step) {
@@ -175,13 +194,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&full[stage], phase, p.wait_limit_ns, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint64_t da = umma_desc_k_sw128(smem_u32(sA + stage * A_STAGE));
-          const uint64_t db = umma_desc_k_sw128(smem_u32(sB + stage * B_STAGE));
+          const uint32_t a_addr = smem_u32(sA + stage * A_STAGE), b_addr = smem_u32(sB + stage * B_STAGE);
+          const uint64_t da = MN && p.a_mn ? umma_desc_mn_sw128(a_addr, MN_BLOCK) : umma_desc_k_sw128(a_addr);
+          const uint64_t db = MN && p.b_mn ? umma_desc_mn_sw128(b_addr, MN_BLOCK) : umma_desc_k_sw128(b_addr);
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
-            // Advancing K inside the 128-byte swizzle atom: +32 bytes = +2 in descriptor address units.
-            if (PAIR) umma_bf16_pair(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-            else umma_bf16(d_tmem, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+            if (PAIR) umma_bf16_pair(d_tmem, da + k * a_step, db + k * b_step, idesc, (kb | k) != 0);
+            else umma_bf16(d_tmem, da + k * a_step, db + k * b_step, idesc, (kb | k) != 0);
           }
           // The stage is free (in both CTAs of a pair) once these MMAs have read it.
           if (PAIR) umma_commit_pair(&empty[stage]);
@@ -405,7 +424,7 @@ static bool pair_wanted() {
 
 using namespace bshmem;
 
-extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stream) {
+static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t stream) {
   if (!a || !a->A || !a->B || !a->out || !a->error_flag) return BSHMEM_FUSED_ERR_ARGS;
   const int npes = a->npes, mode = a->mode;
   if (npes < 1 || npes > BSHMEM_FUSED_MAX_PES || a->rank < 0 || a->rank >= npes) return BSHMEM_FUSED_ERR_ARGS;
@@ -430,7 +449,10 @@ extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stre
   // A pair takes two consecutive 128-row tiles of one PE's block of rows.
   bool pair = pair_wanted() && rows_per_pe % (2 * BM) == 0 && grid >= 2 && !grouped;  // ragged groups do not pair up
   if (pair) grid &= ~1;
-  int st = make_map(&p.tmA, a->A, a->M, a->K, BM);
+  p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
+  p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
+  if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (grouped && layout) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
+  int st = p.a_mn ? make_map(&p.tmA, a->A, a->K, a->M, BK) : make_map(&p.tmA, a->A, a->M, a->K, BM);
   if (st) return st;
   const bool reduce_mode = (mode == BSHMEM_FUSED_RS || mode == BSHMEM_FUSED_AR) && npes > 1;
   if (mode == BSHMEM_FUSED_AR && npes > 1) {
@@ -494,42 +516,42 @@ extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stre
     p.group_n = a->N;
     p.out_local = (char*)a->out;
   }
-  st = make_map(&p.tmB, a->B, grouped ? (uint64_t)a->groups * a->N : (uint64_t)a->N, a->K, pair ? BN / 2 : BN);
+  if (p.b_mn) st = make_map(&p.tmB, a->B, a->K, a->N, BK);
+  else st = make_map(&p.tmB, a->B, grouped ? (uint64_t)a->groups * a->N : (uint64_t)a->N, a->K, pair ? BN / 2 : BN);
   if (st) return st;
+  static void (*const kernels[4])(FusedParams) = {gemm_fused_kernel<false, false>, gemm_fused_kernel<false, true>, gemm_fused_kernel<true, false>, gemm_fused_kernel<true, true>};
   if (g_attr_set_for_device != device) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) {
-      fprintf(stderr, "bshmem_fused_gemm: cannot reserve %d bytes of shared memory: %s\n", SMEM_BYTES, cudaGetErrorString(e));
-      return BSHMEM_FUSED_ERR_DRIVER;
+    for (auto k : kernels) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+      if (e != cudaSuccess) {
+        fprintf(stderr, "bshmem_fused_gemm: cannot reserve %d bytes of shared memory: %s\n", SMEM_BYTES, cudaGetErrorString(e));
+        return BSHMEM_FUSED_ERR_DRIVER;
+      }
     }
     g_attr_set_for_device = device;
   }
-  cudaError_t e;
-  if (pair) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, gemm_fused_kernel<true>, p);
-  } else {
-    gemm_fused_kernel<false><<<grid, NTHREADS, SMEM_BYTES, stream>>>(p);
-    e = cudaGetLastError();
-  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pair ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[(pair ? 2 : 0) + (layout ? 1 : 0)], p);
   if (e != cudaSuccess) {
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
     return BSHMEM_FUSED_ERR_DRIVER;
   }
   return 0;
 }
+
+extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stream) { return launch_gemm(a, 0, stream); }
+extern "C" int bshmem_fused_gemm_layout(const bshmem_fused_args_t* a, int layout, cudaStream_t stream) { return launch_gemm(a, layout, stream); }
 
 extern "C" int bshmem_fused_gemm_smem_bytes(void) { return SMEM_BYTES; }
 

@@ -51,6 +51,7 @@ struct alignas(64) FusedParams {
   const int* group_offsets;                  // GROUPED: device array [groups + 1], rows of group g are [offsets[g], offsets[g + 1])
   int groups, group_n;                       // GROUPED: number of groups; rows of B (output columns) per group
   int red_rows;                              // switch path: rows per work item of the reducing warps (16 or 32)
+  int a_mn, b_mn;                            // operand is stored with K outermost ([K][M] / [K][N]): loaded as it lies, no transpose pass
   int sw_reduce;                             // RS/AR: partial tiles stay local and the owner fetches their sum through the switch
 };
 

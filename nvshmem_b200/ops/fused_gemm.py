@@ -54,6 +54,8 @@ def fused_lib() -> C.CDLL:
         _lib = C.CDLL(str(path))
         _lib.bshmem_fused_gemm.restype = C.c_int
         _lib.bshmem_fused_gemm.argtypes = [C.POINTER(_Args), C.c_void_p]
+        _lib.bshmem_fused_gemm_layout.restype = C.c_int
+        _lib.bshmem_fused_gemm_layout.argtypes = [C.POINTER(_Args), C.c_int, C.c_void_p]
     return _lib
 
 
@@ -88,16 +90,16 @@ def take_error(device=None) -> int:
     return v
 
 
-def _launch(args: _Args, stream) -> None:
-    st = fused_lib().bshmem_fused_gemm(C.byref(args), C.c_void_p(stream))
+def _launch(args: _Args, stream, x_t: bool = False, w_t: bool = False) -> None:
+    st = fused_lib().bshmem_fused_gemm_layout(C.byref(args), int(x_t) + 2 * int(w_t), C.c_void_p(stream))
     if st != 0:
         raise FusedGemmError(f"bshmem_fused_gemm: {_ERRORS.get(st, st)}")
 
 
-def _check_operands(x: torch.Tensor, w: torch.Tensor) -> None:
+def _check_operands(x: torch.Tensor, w: torch.Tensor, x_t: bool = False, w_t: bool = False) -> None:
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise FusedGemmError("operands must be bfloat16")
-    if x.dim() != 2 or w.dim() != 2 or x.shape[1] != w.shape[1]:
+    if x.dim() != 2 or w.dim() != 2 or x.shape[0 if x_t else 1] != w.shape[0 if w_t else 1]:
         raise FusedGemmError(f"shape mismatch: x {tuple(x.shape)} w {tuple(w.shape)}")
     if not x.is_contiguous() or not w.is_contiguous():
         raise FusedGemmError("operands must be contiguous")
@@ -108,12 +110,14 @@ def _check_out(out: torch.Tensor, rows: int, cols: int) -> None:
         raise FusedGemmError(f"`out` must be a contiguous, 16-byte aligned bfloat16 tensor of shape {(rows, cols)}")
 
 
-def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, max_ctas: int = 0, act: str | None = None) -> torch.Tensor:
+def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, max_ctas: int = 0, act: str | None = None, x_t: bool = False,
+         w_t: bool = False) -> torch.Tensor:
     """``act(x[M,K] @ w[N,K].T)`` -> bf16 ``[M,N]`` on the tcgen05/TMEM kernel; ``act`` is None or ``"gelu_tanh"``
-    (applied to the fp32 accumulators in the epilogue)."""
-    _check_operands(x, w)
-    M, K = x.shape
-    N = w.shape[0]
+    (applied to the fp32 accumulators in the epilogue).  ``x_t`` / ``w_t``: the operand is stored transposed, ``x[K,M]`` /
+    ``w[K,N]`` (contiguous); the kernel reads it as it lies."""
+    _check_operands(x, w, x_t, w_t)
+    K, M = x.shape if x_t else x.shape[::-1]
+    N = w.shape[1 if w_t else 0]
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     else:
@@ -124,7 +128,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, max_
     a.M, a.N, a.K, a.rank, a.npes, a.mode = M, N, K, 0, 1, MODES["plain"]
     a.epoch, a.max_ctas = 1, max_ctas
     a.error_flag = _error_flag(x.device).data_ptr()
-    _launch(a, torch.cuda.current_stream().cuda_stream)
+    _launch(a, torch.cuda.current_stream().cuda_stream, x_t, w_t)
     return out
 
 
@@ -235,9 +239,10 @@ class GemmReduceScatter:
             core.barrier_all()
             torch.cuda.synchronize()
 
-    def forward(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
-        _check_operands(x, w)
-        if x.shape[0] != self.M or w.shape[0] != self.N:
+    def forward(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, w_t: bool = False) -> torch.Tensor:
+        """``w_t``: the weight is stored as ``[K_local, N]``."""
+        _check_operands(x, w, w_t=w_t)
+        if x.shape[0] != self.M or w.shape[1 if w_t else 0] != self.N:
             raise FusedGemmError("operand shapes differ from the ones this object was built for")
         if out is None:
             out = self.out
@@ -264,7 +269,7 @@ class GemmReduceScatter:
                 a.flags_peer[q] = self._peer[q][1]
                 a.out_peer[q] = self._peer[q][2]
             a.out_mc = self._out_mc
-        _launch(a, torch.cuda.current_stream().cuda_stream)
+        _launch(a, torch.cuda.current_stream().cuda_stream, w_t=w_t)
         if self.mode == "ar" and self.npes > 1:
             # Tiles written by the other PEs are complete once everyone's kernel has ended.
             self.core.barrier_all(stream=torch.cuda.current_stream())
@@ -329,11 +334,12 @@ class AllGatherGemm:
         self.shard = self.gathered[self.rank * self.rows:(self.rank + 1) * self.rows]
         self.out = None
 
-    def forward(self, w: torch.Tensor, out: torch.Tensor | None = None, act: str | None = None) -> torch.Tensor:
+    def forward(self, w: torch.Tensor, out: torch.Tensor | None = None, act: str | None = None, w_t: bool = False) -> torch.Tensor:
         """``act(gathered @ w.T)``.  Without ``out=`` the result tensor is owned by the object and overwritten by the
-        next call; ``act`` is None or ``"gelu_tanh"`` (fused into the epilogue)."""
-        _check_operands(self.gathered, w)
-        N = w.shape[0]
+        next call; ``act`` is None or ``"gelu_tanh"`` (fused into the epilogue).  ``w_t``: the weight is stored as
+        ``[K, N_local]``."""
+        _check_operands(self.gathered, w, w_t=w_t)
+        N = w.shape[1 if w_t else 0]
         if out is None:
             if self.out is None or self.out.shape[1] != N:
                 self.out = torch.empty(self.M, N, dtype=torch.bfloat16, device=self.device)
@@ -367,7 +373,7 @@ class AllGatherGemm:
                     lib.nvshmemx_putmem_signal_on_stream(C.c_void_p(shard_ptr), C.c_void_p(shard_ptr), shard_bytes, C.c_void_p(flag_ptr), self.epoch, 9,
                                                          (self.rank + o) % self.npes, C.c_void_p(self._comm.cuda_stream))
                 self._sent.record(self._comm)
-        _launch(a, torch.cuda.current_stream().cuda_stream)
+        _launch(a, torch.cuda.current_stream().cuda_stream, w_t=w_t)
         if self.npes > 1 and self.copy_engine:
             torch.cuda.current_stream().wait_event(self._sent)  # the shard may be rewritten once the copies have read it
         return out

@@ -47,8 +47,10 @@ class _OpCache:
         self.ag.clear()
 
 
-def _t(x: torch.Tensor) -> torch.Tensor:
-    return x.t().contiguous()
+def _aligned(x: torch.Tensor) -> torch.Tensor:
+    """`x` as a contiguous tensor whose storage starts on the 16-byte boundary that the kernel's loads need."""
+    x = x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
 
 
 class _ColumnParallelFn(torch.autograd.Function):
@@ -69,11 +71,11 @@ class _ColumnParallelFn(torch.autograd.Function):
         (weight,) = ctx.saved_tensors
         dy = dy.contiguous()
         x_full = ctx.x_full
-        # dW[Nl, K] = dY^T @ X_full
-        dw = fg.gemm(_t(dy), _t(x_full))
+        # dW[Nl, K] = dY^T @ X_full, both operands read as they lie (tokens outermost)
+        dw = fg.gemm(_aligned(dy), x_full, x_t=True, w_t=True)
         # dX_shard[M/n, K] = reduce_scatter(dY[M, Nl] @ W[Nl, K])
         rs = ctx.cache.reduce_scatter(ctx.M, ctx.K)
-        dx = rs(dy, _t(weight), out=torch.empty(rs.rows, ctx.K, dtype=torch.bfloat16, device=dy.device))
+        dx = rs(dy, _aligned(weight), out=torch.empty(rs.rows, ctx.K, dtype=torch.bfloat16, device=dy.device), w_t=True)
         return dx, dw, None, None, None
 
 
@@ -93,10 +95,9 @@ class _RowParallelFn(torch.autograd.Function):
         # dX[M, Kl] = all_gather(dY_shard)[M, N] @ W[N, Kl]
         ag = ctx.cache.all_gather(ctx.M, ctx.N)
         ag.shard.copy_(dy_shard)
-        wt = _t(weight)
-        dx = ag(wt, out=torch.empty(ctx.M, wt.shape[0], dtype=torch.bfloat16, device=dy_shard.device))
+        dx = ag(_aligned(weight), out=torch.empty(ctx.M, weight.shape[1], dtype=torch.bfloat16, device=dy_shard.device), w_t=True)
         # dW[N, Kl] = dY_full^T @ X
-        dw = fg.gemm(_t(ag.gathered), _t(x))
+        dw = fg.gemm(ag.gathered, _aligned(x), x_t=True, w_t=True)
         return dx, dw, None
 
 

@@ -97,3 +97,21 @@ def test_interleave_gate_up_orders_rows_in_blocks_of_32():
     w = torch.arange(2 * F, dtype=torch.float32).view(2 * F, 1).expand(2 * F, K).contiguous()
     r = fg.interleave_gate_up(w)[:, 0].tolist()
     assert r[:32] == list(range(0, 32)) and r[32:64] == list(range(F, F + 32)) and r[64:96] == list(range(32, 64)) and r[96:] == list(range(F + 32, 2 * F))
+
+
+@pytest.mark.parametrize("x_t,w_t", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 64), (384, 512, 192), (256, 256, 64), (512, 1280, 1088)])
+def test_gemm_reads_transposed_operands_as_they_lie(M, N, K, x_t, w_t):
+    """Operands stored with K outermost, for one CTA per tile (odd number of 128-row blocks) and for CTA pairs: the same
+    MMAs on the same values in the same order, so the result equals the one of the K-major operands bit by bit."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    got = fg.gemm(x.t().contiguous() if x_t else x, w.t().contiguous() if w_t else w, x_t=x_t, w_t=w_t)
+    want = fg.gemm(x, w)
+    torch.cuda.synchronize()
+    fg.check_errors()
+    assert torch.equal(got, want)
+    ref = _ref(x, w)
+    assert (got.float() - ref).abs().max().item() <= ref.abs().max().item() * 2 ** -7 + 1e-3
