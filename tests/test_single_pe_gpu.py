@@ -65,6 +65,25 @@ def test_collectives_on_one_pe_are_copies(nv, dtype):
     nv.free_tensor(dst)
 
 
+@pytest.mark.parametrize("n,so,do", [(1, 0, 0), (15, 0, 0), (16384, 0, 0), (16401, 0, 0), ((1 << 25) + 3, 16, 16), (40000, 8, 16), (40002, 4, 12), (40001, 2, 6), (70001, 1, 4)])
+def test_collectives_of_one_member_copy_every_byte_and_no_more(nv, n, so, do):
+    """Tails, all alignments of the two addresses, one and several rounds of the copy kernel; nothing outside is written."""
+    src = nv.tensor((n + 64,), torch.uint8)
+    dst = nv.tensor((n + 64,), torch.uint8)
+    src.copy_(torch.randint(0, 256, (n + 64,), device="cuda", dtype=torch.uint8))
+    for coll in ("reduce", "reducescatter", "fcollect", "alltoall", "broadcast"):
+        dst.fill_(7)
+        nv.collective_on_buffer(coll, 0, dst[do:do + n], src[so:so + n], op="sum")
+        torch.cuda.synchronize()
+        assert torch.equal(dst[do:do + n], src[so:so + n]), coll
+        assert bool((dst[:do] == 7).all()) and bool((dst[do + n:] == 7).all()), coll
+        nv.collective_on_buffer(coll, 0, dst[do:do + n], dst[do:do + n], op="sum")  # in place
+    torch.cuda.synchronize()
+    assert torch.equal(dst[do:do + n], src[so:so + n]) and nv.error_bits() == 0
+    nv.free_tensor(src)
+    nv.free_tensor(dst)
+
+
 def test_signal_and_wait_on_stream(nv):
     sig = nv.tensor((1,), torch.int64, zero=True)
     nv.signal_op(sig, 5, nv.SignalOp.SIGNAL_SET, 0)
