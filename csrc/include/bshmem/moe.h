@@ -4,7 +4,7 @@
 // (expert e lives on PE e / (E/npes)).  One cooperative kernel counts, exchanges the counts with
 // all PEs, derives where each (token, expert) pair lands and pushes the rows straight into the
 // receive buffer of the owning PE, grouped by expert, then by source PE.  The rows travel as bf16
-// or as fp8 e4m3 with one fp32 scale per 128 values (quantised on the fly).
+// or as fp8 e4m3 with one fp32 scale per 128 values (quantised on the fly).  One PE (without dup_src) runs one or two plain kernels instead.
 // combine: the inverse; every PE pulls, for each of its tokens, the K expert outputs from the PEs
 // that own them and writes their weighted sum.
 // The library allocates nothing: receive buffers, the count matrix and the flags are symmetric

@@ -154,6 +154,82 @@ def test_moe_dispatch_combine_single_pe(nv):
     W._moe_check(nv, "fp8", T=128, H=1024, K=8, E=32, seed=12)
 
 
+@pytest.mark.parametrize("payload", [0, 1])
+@pytest.mark.parametrize("T,H,K,E,cap", [(1, 128, 1, 1, 0), (3, 640, 16, 1024, 0), (128, 256, 16, 64, 0), (2049, 128, 1, 7, 0), (683, 2176, 3, 5, 0),
+                                         (700, 2304, 8, 256, 0), (9000, 384, 9, 1000, 0), (100, 256, 4, 8, 77), (1000, 1152, 8, 8, 5000), (5, 16512, 2, 4, 0)])
+def test_local_dispatch_agrees_with_the_general_one(T, H, K, E, cap, payload):
+    """One PE without `dup_src` takes the kernels that meet nobody (one for up to 2048 pairs, two above); with `dup_src` the
+    general kernel runs.  Offsets, counts and the multiset of rows per expert must be the same, and every row must hold what its slot
+    says, to the byte; too small a buffer drops the rows beyond it and sets the overflow bit."""
+    import ctypes as C
+    from nvshmem_b200.ops.moe import _lib, _DispatchArgs
+    lib = _lib()
+    torch.manual_seed(T + H + K + E)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    x[0, :128] = 0
+    idx = torch.randint(-1, E + 1, (T, K), device="cuda", dtype=torch.int32)  # -1 and E are dropped
+    cap = cap or T * K
+    res = []
+    for general in (False, True):
+        z = lambda *s, dt=torch.int32, v=0: torch.full(s, v, dtype=dt, device="cuda")
+        recv = z(cap + 1, H if payload else 2 * H, dt=torch.uint8, v=9)
+        scale, slot, offs, src = z(cap + 1, H // 128, dt=torch.float32, v=9), z(T, K, v=-7), z(E + 1, v=-7), z(E, 1, v=-7)
+        counts, flags, scratch, err, dup = z(E, v=-7), z(4, dt=torch.int64), z(lib.bshmem_moe_scratch_bytes(E) // 4 + 64), z(1), z(cap)
+        a = _DispatchArgs()
+        a.T, a.H, a.K, a.E, a.rank, a.npes, a.payload, a.cap_rows, a.epoch = T, H, K, E, 0, 1, payload, cap, 1
+        a.error_flag, a.x, a.topk_idx = err.data_ptr(), x.data_ptr(), idx.data_ptr()
+        a.recv_x[0], a.recv_scale[0], a.counts[0], a.flags[0] = recv.data_ptr(), scale.data_ptr(), counts.data_ptr(), flags.data_ptr()
+        a.slot_map, a.expert_offsets, a.src_offsets, a.scratch = slot.data_ptr(), offs.data_ptr(), src.data_ptr(), scratch.data_ptr()
+        if general:
+            a.dup_src[0] = dup.data_ptr()
+        assert lib.bshmem_moe_dispatch(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        assert bool((recv[cap] == 9).all()) and bool((scale[cap] == 9).all()), "written past the buffer"
+        res.append((recv, scale, slot, offs, src, counts, int(err)))
+    local, general = res
+    valid = (idx >= 0) & (idx < E)
+    for k in (3, 4, 5):
+        assert torch.equal(local[k], general[k])
+    total = int(valid.sum())
+    assert int(local[3][E]) == total and local[6] == (2 if total > cap else 0) and local[6] == general[6]
+    got = local[2].long()
+    assert bool((got[~valid] == -1).all()) and int((got >= 0).sum()) == min(total, cap)
+    t, k = (got >= 0).nonzero(as_tuple=True)
+    rows, e = got[t, k], idx[t, k].long()
+    assert torch.equal(rows.sort().values, torch.arange(rows.numel(), device="cuda"))
+    assert bool(((rows >= local[3].long()[e]) & (rows < local[3].long()[e + 1])).all())
+    if payload:  # the general kernel's bytes for the same token, wherever that one put it
+        tg, kg = (general[2] >= 0).nonzero(as_tuple=True)
+        q, s = torch.zeros(T, H, dtype=torch.uint8, device="cuda"), torch.zeros(T, H // 128, device="cuda")
+        q[tg], s[tg] = general[0][general[2].long()[tg, kg]], general[1][general[2].long()[tg, kg]]
+        seen = torch.zeros(T, dtype=torch.bool, device="cuda")
+        seen[tg] = True
+        keep = seen[t]
+        assert torch.equal(local[0][rows][keep], q[t][keep]) and torch.equal(local[1][rows][keep], s[t][keep])
+    else:
+        assert torch.equal(local[0][rows].view(torch.bfloat16), x[t])
+
+
+@pytest.mark.parametrize("T,H,K", [(1, 128, 1), (3, 640, 16), (61, 7168, 8), (295, 256, 9), (1500, 384, 4)])
+def test_local_combine_over_column_ranges(nv, T, H, K):
+    """Few tokens: a token's row is cut into column ranges for several CTAs.  fp32 sums of K products, one rounding to bf16."""
+    from nvshmem_b200.ops.moe import MoeDispatchCombine
+    torch.manual_seed(T + H + K)
+    moe = MoeDispatchCombine(T, H, K, 32)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    w = torch.rand(T, K, device="cuda")
+    idx = torch.rand(T, 32, device="cuda").topk(K, dim=-1).indices.to(torch.int32).contiguous()
+    idx[T // 2, K - 1] = -1
+    recv, _ = moe.dispatch(x, idx)
+    moe.expert_out.copy_(recv)
+    want = x.double() * (w * (idx >= 0)).double().sum(-1, keepdim=True)
+    got = moe.combine(idx, w).double()
+    # one rounding to bf16 (8 significant bits: half a unit in the last place is at most 2^-8 of the value) and the rounding
+    # of K fp32 products and sums, all of one sign
+    assert bool(((got - want).abs() <= want.abs() * (2.0 ** -8 + 2 * K * 2.0 ** -24) + 1e-30).all())
+    moe.close()
+
+
 @pytest.mark.parametrize("payload,tol", [("bf16", 0.03), ("fp8", 0.08)])
 def test_moe_block_matches_fp32_reference_single_pe(nv, payload, tol):
     """Router + dispatch + expert MLPs + combine against a plain PyTorch fp32 version of the same block."""
