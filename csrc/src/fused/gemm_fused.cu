@@ -27,7 +27,7 @@
 //            a flag write per shard; no SM takes part) or by the auxiliary warps of all CTAs (a counter per 128-row
 //            block); the producer warp consumes shards in arrival order (own, then rank-1, rank-2, …) and only waits
 //            when one has not landed.  Remote data is always read from this GPU's own memory.
-//   MODE_PLAIN  no collective (also what 1 PE runs).
+//   MODE_PLAIN  no collective (also what 1 PE runs; products of few tiles go to gemm_split_kernel, see gemm_split.cuh).
 // Every wait (mbarrier, flag) is bounded; on expiry the CTA unwinds, frees its tensor memory and sets `error_flag`.
 // No load uses a cluster-wide broadcast form, so the same binary runs on any number of GPUs.
 // (reference for the capability: examples/gemm_allreduce/*, which fuses a CUTLASS GEMM with an NVLS allreduce)
@@ -44,6 +44,7 @@
 
 
 #include "gemm_fused_common.cuh"
+#include "gemm_split.cuh"
 
 namespace bshmem {
 using namespace sm100;
@@ -420,6 +421,76 @@ static bool pair_wanted() {
   return on;
 }
 
+// The tile width and the number of K parts for `tiles` output tiles of 128 x 256, if one wave of CTAs can hold them.  A model
+// of measured times (us): a fixed part (launch, first loads, reduction through the cluster, store) and, per 64-wide K step,
+// the time an SM needs to load a stage (about 70 bytes per clock whatever the tile), or that of all the bytes from HBM.
+//   128 x 512 x 512     64/1 4.6   64/4 5.3   128/1 5.5   256/1 7.7    (persistent kernel 8.0)
+//   128 x 1024 x 2048   64/1 7.8   64/4 6.2   128/4 7.4   256/4 10.4   (14.9)
+//   128 x 3584 x 8192   64/2 17.1  128/2 21.3  128/4 16.8  256/4 22.6  (52.0)
+//   512 x 3584 x 8192   128/1 31.8  256/2 32.7                         (43.4)
+// Clusters of eight find too few places when there are many (16 of them ran in two waves), clusters of four find 32.
+struct SplitPlan {
+  int n_tile, splits;
+  double us;
+};
+static SplitPlan plan_split(int tiles, int kblocks, double bytes, int sms) {
+  static const int width[3] = {64, 128, 256};
+  static const double fixed[3][4] = {{3.7, 5.1, 5.2, 5.3}, {4.4, 6.4, 6.0, 6.4}, {5.5, 8.4, 8.0, 8.7}}, step[3] = {0.14, 0.20, 0.36};
+  SplitPlan best = {0, 0, 0.0};
+  for (int w = 0; w < 3; ++w)
+    for (int l = 0; l < 4; ++l) {
+      const int splits = 1 << l, most = l == 3 ? sms * 7 / 16 : l == 2 ? sms * 7 / 8 : sms;
+      if ((long)tiles * (BN / width[w]) * splits > most || splits > kblocks) continue;
+      const double loads = ((kblocks + splits - 1) / splits) * step[w], hbm = bytes / 6.2e6;
+      const double us = fixed[w][l] + (loads > hbm ? loads : hbm);
+      if (!best.n_tile || us < best.us) best = {width[w], splits, us};
+    }
+  return best;
+}
+
+// Tiles [first, first + tiles) of the product by gemm_split_kernel.
+static int launch_split(const bshmem_fused_args_t* a, int layout, int first, int tiles, int n_tile, int splits, uint64_t wait_limit_ns, cudaStream_t stream) {
+  SplitParams p;
+  memset(&p, 0, sizeof(p));
+  p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
+  p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
+  int st = p.a_mn ? make_map(&p.tmA, a->A, a->K, a->M, BK) : make_map(&p.tmA, a->A, a->M, a->K, BM);
+  if (!st) st = p.b_mn ? make_map(&p.tmB, a->B, a->K, a->N, BK) : make_map(&p.tmB, a->B, a->N, a->K, n_tile);
+  if (!st && ((uintptr_t)a->out & 15)) st = BSHMEM_FUSED_ERR_ALIGNMENT;
+  if (st) return st;
+  p.out = (char*)a->out;
+  p.error_flag = a->error_flag;
+  p.wait_limit_ns = wait_limit_ns;
+  p.M = a->M; p.N = a->N; p.K = a->K; p.act = a->act;
+  p.first_tile = first;
+  p.splits = splits;
+  static void (*const kernels[6])(SplitParams) = {gemm_split_kernel<64, false>, gemm_split_kernel<64, true>, gemm_split_kernel<128, false>, gemm_split_kernel<128, true>,
+                                                  gemm_split_kernel<256, false>, gemm_split_kernel<256, true>};
+  const int which = (n_tile == 64 ? 0 : n_tile == 128 ? 2 : 4) + (layout ? 1 : 0);
+  cudaError_t e = cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM);
+  if (e != cudaSuccess) return BSHMEM_FUSED_ERR_DRIVER;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles * (BN / n_tile) * splits);
+  cfg.blockDim = dim3(SPLIT_THREADS);
+  cfg.dynamicSmemBytes = SPLIT_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 2 : 1;
+  e = cudaLaunchKernelEx(&cfg, kernels[which], p);
+  if (e != cudaSuccess) {
+    fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
+    return BSHMEM_FUSED_ERR_DRIVER;
+  }
+  return 0;
+}
+
 }  // namespace bshmem
 
 using namespace bshmem;
@@ -441,7 +512,6 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   p.wait_limit_ns = a->wait_limit_ms ? (uint64_t)a->wait_limit_ms * 1000000ull : 10000000000ull;
   p.error_flag = a->error_flag;
   const int rows_per_pe = a->M / npes;
-  const int tmr = rows_per_pe / BM;
   int device = 0, sms = 0;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -452,6 +522,13 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
   p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
   if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (grouped && layout) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
+  if (npes == 1 && !grouped && grid == sms) {
+    const int tiles = (a->M / BM) * (a->N / BN), kblocks = a->K / BK;
+    const SplitPlan plan = plan_split(tiles, kblocks, 2.0 * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N), sms);
+    // The persistent kernel: 6 us for launch, first loads and epilogue, then 0.29 us (pairs) or 0.36 us per K step and wave.
+    const double here = 6.0 + (double)((tiles + sms - 1) / sms) * kblocks * (pair ? 0.29 : 0.36);
+    if (plan.n_tile && plan.us < 0.97 * here) return launch_split(a, layout, 0, tiles, plan.n_tile, plan.splits, p.wait_limit_ns, stream);
+  }
   int st = p.a_mn ? make_map(&p.tmA, a->A, a->K, a->M, BK) : make_map(&p.tmA, a->A, a->M, a->K, BM);
   if (st) return st;
   const bool reduce_mode = (mode == BSHMEM_FUSED_RS || mode == BSHMEM_FUSED_AR) && npes > 1;
@@ -563,6 +640,13 @@ extern "C" int bshmem_fused_test_ag_units(int K, int grid, int* out) {
   out[0] = u.unit_bytes;
   out[1] = u.units_per_block;
   return 0;
+}
+
+// Test hook (host only): what plan_split chooses; out = {tile width (0: the persistent kernel), K parts}.
+extern "C" void bshmem_fused_test_split_plan(int tiles, int kblocks, double bytes, int sms, int* out) {
+  const SplitPlan plan = plan_split(tiles, kblocks, bytes, sms);
+  out[0] = plan.n_tile;
+  out[1] = plan.splits;
 }
 
 // Test hook (host only): the tile that position `t` of the tile order names, for the checks of the order's

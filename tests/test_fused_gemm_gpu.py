@@ -115,3 +115,28 @@ def test_gemm_reads_transposed_operands_as_they_lie(M, N, K, x_t, w_t):
     assert torch.equal(got, want)
     ref = _ref(x, w)
     assert (got.float() - ref).abs().max().item() <= ref.abs().max().item() * 2 ** -7 + 1e-3
+
+
+@pytest.mark.parametrize("act", [None, "gelu_tanh"])
+@pytest.mark.parametrize("M,N,K", [(128, 256, 64), (128, 256, 128), (128, 1024, 2048), (256, 512, 8192), (128, 3584, 8128), (384, 1536, 704), (512, 3584, 1984), (1152, 2816, 192),
+                                   (128, 8192, 3584), (1280, 2816, 1984)])
+def test_products_of_few_tiles(M, N, K, act):
+    """Narrow tiles with K divided over a cluster (1 to 8 parts, even and uneven), the single wave it has to fit and the persistent
+    kernel beyond.  fp32 sums in another order differ by about sqrt(K) 2^-24 of the operands' scale, far below the
+    rounding to bf16 (2^-8 of the value at most)."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    room = 1e-4 * want.abs().max()
+    if act:
+        # the hardware tanh is good to 2^-10.99 relative; its share of x is at most half of that
+        room = room + want.abs() * 2 ** -11
+        want = torch.nn.functional.gelu(want, approximate="tanh")
+    for x_t, w_t in ((False, False), (True, True), (False, True)):
+        got = fg.gemm(x.t().contiguous() if x_t else x, w.t().contiguous() if w_t else w, act=act, x_t=x_t, w_t=w_t)
+        torch.cuda.synchronize()
+        fg.check_errors()
+        assert bool(((got.double() - want).abs() <= want.abs() * 2 ** -8 + room).all()), (x_t, w_t)
+    assert torch.equal(fg.gemm(x, w, act=act), fg.gemm(x, w, act=act))
