@@ -38,10 +38,8 @@
 #include <stdio.h>
 #include <stdlib.h>
 
-#include <map>
+#include <atomic>
 #include <mutex>
-#include <tuple>
-
 
 #include "gemm_fused_common.cuh"
 #include "gemm_split.cuh"
@@ -467,8 +465,15 @@ static int launch_split(const bshmem_fused_args_t* a, int layout, int first, int
   static void (*const kernels[6])(SplitParams) = {gemm_split_kernel<64, false>, gemm_split_kernel<64, true>, gemm_split_kernel<128, false>, gemm_split_kernel<128, true>,
                                                   gemm_split_kernel<256, false>, gemm_split_kernel<256, true>};
   const int which = (n_tile == 64 ? 0 : n_tile == 128 ? 2 : 4) + (layout ? 1 : 0);
-  cudaError_t e = cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM);
-  if (e != cudaSuccess) return BSHMEM_FUSED_ERR_DRIVER;
+  static std::atomic<uint64_t> ready[6];  // per kernel: the GPUs (bit = ordinal) whose shared-memory limit is set
+  int device = 0;
+  cudaGetDevice(&device);
+  cudaError_t e = cudaSuccess;
+  if (device >= 64 || !(ready[which].load(std::memory_order_acquire) >> device & 1)) {
+    e = cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM);
+    if (e != cudaSuccess) return BSHMEM_FUSED_ERR_DRIVER;
+    if (device < 64) ready[which].fetch_or(1ull << device, std::memory_order_release);
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * (BN / n_tile) * splits);
   cfg.blockDim = dim3(SPLIT_THREADS);

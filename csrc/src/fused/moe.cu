@@ -29,6 +29,10 @@
 #include <limits.h>
 #include <string.h>
 
+#include <map>
+#include <mutex>
+#include <tuple>
+
 #include "../../include/bshmem/moe.h"
 #include "../../include/bshmem/tcgen05.cuh"
 
@@ -755,15 +759,26 @@ __global__ void __launch_bounds__(THREADS) push_rows_fp8_kernel(const __grid_con
 
 static size_t dispatch_smem(int E, int) { return (size_t)E * 8 + 16; }  // two int arrays of E entries; rows go through registers
 
-// Cooperative grid: as many CTAs as are co-resident, at most one per token.
+// CTAs of a kernel that are co-resident on the current GPU, 0 on an error.  Asked once per kernel, launch shape and GPU: the
+// driver's answer takes longer than the rest of a small launch.
+static int resident_ctas(const void* k, size_t smem, int threads) {
+  static std::mutex mutex;
+  static std::map<std::tuple<const void*, size_t, int, int>, int> known;
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  int& n = known[std::make_tuple(k, smem, threads, dev)];
+  if (n) return n;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) return 0;
+  return n = per_sm * sms;
+}
+// Grid: as many CTAs as are co-resident (what a cooperative launch allows), at most `want`.
 template <class Kernel>
 static int coop_grid(Kernel k, size_t smem, int want, int max_ctas, int* grid_out, int threads = THREADS) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return BSHMEM_MOE_ERR_DRIVER;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess || per_sm < 1) return BSHMEM_MOE_ERR_DRIVER;
-  int grid = per_sm * sms;
+  int grid = resident_ctas((const void*)k, smem, threads);
+  if (grid < 1) return BSHMEM_MOE_ERR_DRIVER;
   if (grid > want) grid = want;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
   if (grid < 1) grid = 1;

@@ -32,6 +32,15 @@ OP_AND, OP_OR, OP_XOR, OP_MIN, OP_MAX, OP_SUM, OP_PROD = range(7)
 ERR_WAIT_TIMEOUT, ERR_BAD_PE, ERR_BAD_ADDRESS, ERR_SCRATCH_TOO_SMALL, ERR_GLOBAL_EXIT, ERR_BAD_TEAM = 1, 2, 4, 8, 16, 32
 
 
+def current_stream_handle() -> int:
+    """Handle of the current torch stream of the current device, 0 without a GPU.  Every stream-ordered call asks for it, and
+    building the ``torch.cuda.Stream`` object that carries it takes 3 us; the handle alone takes 0.2."""
+    import torch
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return int(torch.cuda.current_stream().cuda_stream) if torch.cuda.is_available() else 0
+
+
 class UniqueId(C.Structure):
     _fields_ = [("version", C.c_int), ("internal", C.c_char * 124)]
 

@@ -3,6 +3,7 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 from ..bindings import host as H
 from .memory import tensor_ptr
@@ -15,13 +16,19 @@ RS_ALGOS = {"auto": 0, "pull": 1, "nvls": 2}
 BCAST_ALGOS = {"auto": 0, "push": 1, "ll": 2, "nvls": 3, "pull": 4}
 
 
-def _dtype_code(t) -> int:
+@functools.cache
+def _dtype_table() -> dict:
     import torch
     table = {torch.int8: H.DT_I8, torch.uint8: H.DT_U8, torch.int16: H.DT_I16, torch.int32: H.DT_I32, torch.int64: H.DT_I64, torch.float16: H.DT_F16,
              torch.bfloat16: H.DT_BF16, torch.float32: H.DT_F32, torch.float64: H.DT_F64}
     for name, code in (("uint16", H.DT_U16), ("uint32", H.DT_U32), ("uint64", H.DT_U64)):
         if hasattr(torch, name):
             table[getattr(torch, name)] = code
+    return table
+
+
+def _dtype_code(t) -> int:
+    table = _dtype_table()
     if t.dtype not in table:
         raise NvshmemInvalid(f"dtype {t.dtype} is not supported by the collectives")
     return table[t.dtype]

@@ -4,6 +4,8 @@ from __future__ import annotations
 
 import enum
 
+from ..bindings import host as H
+
 
 class NvshmemError(RuntimeError):
     """A library call failed; the message names the call and the status code."""
@@ -48,8 +50,7 @@ class NvshmemStream:
 
 def stream_handle(stream) -> int:
     if stream is None:
-        import torch
-        return int(torch.cuda.current_stream().cuda_stream) if torch.cuda.is_available() else 0
+        return H.current_stream_handle()
     if isinstance(stream, NvshmemStream):
         return stream.handle
     if isinstance(stream, int):

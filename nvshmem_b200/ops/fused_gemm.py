@@ -128,7 +128,7 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, max_
     a.M, a.N, a.K, a.rank, a.npes, a.mode = M, N, K, 0, 1, MODES["plain"]
     a.epoch, a.max_ctas = 1, max_ctas
     a.error_flag = _error_flag(x.device).data_ptr()
-    _launch(a, torch.cuda.current_stream().cuda_stream, x_t, w_t)
+    _launch(a, H.current_stream_handle(), x_t, w_t)
     return out
 
 
@@ -163,7 +163,7 @@ def grouped_gemm(x: torch.Tensor, w: torch.Tensor, group_offsets: torch.Tensor, 
     a.epoch = 1
     a.group_offsets, a.groups = group_offsets.data_ptr(), G
     a.error_flag = _error_flag(x.device).data_ptr()
-    _launch(a, torch.cuda.current_stream().cuda_stream)
+    _launch(a, H.current_stream_handle())
     return out
 
 
@@ -269,7 +269,7 @@ class GemmReduceScatter:
                 a.flags_peer[q] = self._peer[q][1]
                 a.out_peer[q] = self._peer[q][2]
             a.out_mc = self._out_mc
-        _launch(a, torch.cuda.current_stream().cuda_stream, w_t=w_t)
+        _launch(a, H.current_stream_handle(), w_t=w_t)
         if self.mode == "ar" and self.npes > 1:
             # Tiles written by the other PEs are complete once everyone's kernel has ended.
             self.core.barrier_all(stream=torch.cuda.current_stream())
@@ -373,7 +373,7 @@ class AllGatherGemm:
                     lib.nvshmemx_putmem_signal_on_stream(C.c_void_p(shard_ptr), C.c_void_p(shard_ptr), shard_bytes, C.c_void_p(flag_ptr), self.epoch, 9,
                                                          (self.rank + o) % self.npes, C.c_void_p(self._comm.cuda_stream))
                 self._sent.record(self._comm)
-        _launch(a, torch.cuda.current_stream().cuda_stream, w_t=w_t)
+        _launch(a, H.current_stream_handle(), w_t=w_t)
         if self.npes > 1 and self.copy_engine:
             torch.cuda.current_stream().wait_event(self._sent)  # the shard may be rewritten once the copies have read it
         return out

@@ -13,6 +13,7 @@ import os
 
 import torch
 
+from ..bindings import host as H
 from .fused_gemm import fused_lib, _error_flag
 
 MAX_PES, MAX_TOPK = 8, 16
@@ -89,6 +90,16 @@ class MoeDispatchCombine:
         ptr = (lambda t, q: core.peer_ptr(t, q)) if sym else (lambda t, q: t.data_ptr())
         self._peers = {q: {"recv": ptr(self.recv_raw, q), "scale": ptr(self.recv_scale, q) if self.fp8 else 0, "y": ptr(self.expert_out, q),
                            "counts": ptr(self.counts, q), "flags": ptr(self.flags, q), "dup": ptr(self.dup_src, q) if self.dedup else 0} for q in range(self.npes)}
+        # What every call passes alike (sizes, the peers' addresses of this object's buffers); a call fills in its own copy.
+        d, c = _DispatchArgs(), _CombineArgs()
+        for q in range(self.npes):
+            d.recv_x[q], d.recv_scale[q], d.dup_src[q] = self._peers[q]["recv"], self._peers[q]["scale"], self._peers[q]["dup"]
+            d.counts[q], d.flags[q] = self._peers[q]["counts"], self._peers[q]["flags"]
+            c.y[q], c.flags[q] = self._peers[q]["y"], self._peers[q]["flags"]
+        for a in (d, c):
+            a.T, a.H, a.K, a.E, a.rank, a.npes = T, H, K, E, self.rank, self.npes
+        d.payload, d.cap_rows = int(self.fp8), self.cap_rows
+        self._dispatch_args, self._combine_args = d, c
         if sym:
             core.barrier_all()
             torch.cuda.synchronize()
@@ -109,18 +120,13 @@ class MoeDispatchCombine:
         if topk_idx.shape != (self.T, self.K) or topk_idx.dtype != torch.int32 or not topk_idx.is_contiguous():
             raise MoeError("topk_idx must be contiguous int32 [T, K]")
         self.epoch += 1
-        a = _DispatchArgs()
-        a.T, a.H, a.K, a.E, a.rank, a.npes = self.T, self.H, self.K, self.E, self.rank, self.npes
-        a.payload, a.cap_rows, a.epoch, a.wait_limit_ms = int(self.fp8), self.cap_rows, self.epoch, self.wait_limit_ms
+        a = _DispatchArgs.from_buffer_copy(self._dispatch_args)
+        a.epoch, a.wait_limit_ms = self.epoch, self.wait_limit_ms
         a.error_flag = _error_flag(self.device).data_ptr()
         a.x, a.topk_idx = x.data_ptr(), topk_idx.data_ptr()
-        for q in range(self.npes):
-            a.recv_x[q], a.recv_scale[q] = self._peers[q]["recv"], self._peers[q]["scale"]
-            a.counts[q], a.flags[q] = self._peers[q]["counts"], self._peers[q]["flags"]
-            a.dup_src[q] = self._peers[q]["dup"]
         a.slot_map, a.expert_offsets, a.src_offsets = self.slot_map.data_ptr(), self.expert_offsets.data_ptr(), self.src_offsets.data_ptr()
         a.scratch = self.scratch.data_ptr()
-        st = _lib().bshmem_moe_dispatch(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        st = _lib().bshmem_moe_dispatch(C.byref(a), C.c_void_p(H.current_stream_handle()))
         if st != 0:
             raise MoeError(f"bshmem_moe_dispatch failed with status {st}")
         return self.recv_x, self.expert_offsets
@@ -128,15 +134,12 @@ class MoeDispatchCombine:
     def combine(self, topk_idx: torch.Tensor, topk_weight: torch.Tensor) -> torch.Tensor:
         if topk_weight.shape != (self.T, self.K) or topk_weight.dtype != torch.float32 or not topk_weight.is_contiguous():
             raise MoeError("topk_weight must be contiguous fp32 [T, K]")
-        a = _CombineArgs()
-        a.T, a.H, a.K, a.E, a.rank, a.npes = self.T, self.H, self.K, self.E, self.rank, self.npes
+        a = _CombineArgs.from_buffer_copy(self._combine_args)
         a.epoch, a.wait_limit_ms = self.epoch, self.wait_limit_ms
         a.error_flag = _error_flag(self.device).data_ptr()
-        for q in range(self.npes):
-            a.y[q], a.flags[q] = self._peers[q]["y"], self._peers[q]["flags"]
         a.topk_idx, a.topk_weight, a.slot_map, a.out = topk_idx.data_ptr(), topk_weight.data_ptr(), self.slot_map.data_ptr(), self.out.data_ptr()
         a.scratch = self.scratch.data_ptr()
-        st = _lib().bshmem_moe_combine(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        st = _lib().bshmem_moe_combine(C.byref(a), C.c_void_p(H.current_stream_handle()))
         if st != 0:
             raise MoeError(f"bshmem_moe_combine failed with status {st}")
         return self.out
