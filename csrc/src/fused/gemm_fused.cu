@@ -118,7 +118,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_n = p.N / BN;
-  const int total_tiles = grouped ? g_prefix[p.groups] : (p.M / BM) * tiles_n;
+  const int total_tiles = grouped ? g_prefix[p.groups] : p.tile_end ? p.tile_end : (p.row_blocks ? p.row_blocks : p.M / BM) * tiles_n;
+  // The kernel for the last tiles needs nothing from this one: its CTAs may take the SMs as they become free.
+  if (p.tile_end) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int kblocks = p.K / BK;
   // Pair: worker u = pair index takes tiles 2u + r, 2(u + workers) + r, …
   const int first = PAIR ? ((int)blockIdx.x & ~1) + (int)cta_rank : (int)blockIdx.x;
@@ -146,14 +148,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, p.wait_limit_ns, abort_flag)) break;
           const uint32_t lead = PAIR ? mapa_u32(smem_u32(&full[stage]), 0) : 0;
-          if (PAIR) mbar_expect_tx_cluster(lead, A_STAGE + B_STAGE);
+          // A block without rows (an odd number of blocks, in pairs): whatever the stage holds goes into accumulator rows that
+          // nobody stores, so nothing is loaded.
+          const bool no_a = PAIR && ti.valid_rows == 0;
+          if (PAIR) mbar_expect_tx_cluster(lead, (no_a ? 0 : A_STAGE) + B_STAGE);
           else mbar_expect_tx(&full[stage], A_STAGE + B_STAGE);
           auto load = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
             if (PAIR) tma_load_2d_pair(dst, map, lead, x, y);
             else tma_load_2d(dst, map, &full[stage], x, y);
           };
           // K-major operand: one box of 64 k x all rows.  MN-major operand: boxes of 64 rows (contiguous) x 64 k.
-          if (MN && p.a_mn) {
+          if (no_a) {
+          } else if (MN && p.a_mn) {
 #pragma unroll
             for (int i = 0; i < BM / 64; ++i) load(sA + stage * A_STAGE + i * MN_BLOCK, &p.tmA, ti.a_row + i * 64, kb * BK);
           } else {
@@ -352,7 +358,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
             const uint4 v = *(const uint4*)(buf + r * 128 + ((j ^ (r & 7)) << 4));
             multimem_st_v4(base + (size_t)r * p.N * 2 + j * 16, v);
           }
-        } else if (issuer) {
+        } else if (issuer && ti.valid_rows) {
           const int x = ti.n_tile * BN + c * EPI_COLS;
           if (sw) {
             tma_store_2d(&p.tmStage, buf, x, ti.m_tile * BM);
@@ -433,7 +439,7 @@ struct SplitPlan {
 };
 static SplitPlan plan_split(int tiles, int kblocks, double bytes, int sms) {
   static const int width[3] = {64, 128, 256};
-  static const double fixed[3][4] = {{3.7, 5.1, 5.2, 5.3}, {4.4, 6.4, 6.0, 6.4}, {5.5, 8.4, 8.0, 8.7}}, step[3] = {0.14, 0.20, 0.36};
+  static const double fixed[3][4] = {{2.6, 4.0, 4.1, 4.3}, {3.4, 5.3, 5.0, 5.4}, {4.5, 7.3, 7.0, 7.7}}, step[3] = {0.14, 0.20, 0.36};
   SplitPlan best = {0, 0, 0.0};
   for (int w = 0; w < 3; ++w)
     for (int l = 0; l < 4; ++l) {
@@ -447,7 +453,11 @@ static SplitPlan plan_split(int tiles, int kblocks, double bytes, int sms) {
 }
 
 // Tiles [first, first + tiles) of the product by gemm_split_kernel.
-static int launch_split(const bshmem_fused_args_t* a, int layout, int first, int tiles, int n_tile, int splits, uint64_t wait_limit_ns, cudaStream_t stream) {
+// `row_blocks`: of the tile order (may be one more than there are rows for).  `follows`: the launch before it on the stream is
+// the persistent kernel of the same product.
+static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks, int first, int tiles, bool follows, SplitPlan plan, uint64_t wait_limit_ns,
+                        cudaStream_t stream) {
+  const int n_tile = plan.n_tile, splits = plan.splits;
   SplitParams p;
   memset(&p, 0, sizeof(p));
   p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
@@ -461,6 +471,8 @@ static int launch_split(const bshmem_fused_args_t* a, int layout, int first, int
   p.wait_limit_ns = wait_limit_ns;
   p.M = a->M; p.N = a->N; p.K = a->K; p.act = a->act;
   p.first_tile = first;
+  p.row_blocks = row_blocks;
+  p.follows = follows;
   p.splits = splits;
   static void (*const kernels[6])(SplitParams) = {gemm_split_kernel<64, false>, gemm_split_kernel<64, true>, gemm_split_kernel<128, false>, gemm_split_kernel<128, true>,
                                                   gemm_split_kernel<256, false>, gemm_split_kernel<256, true>};
@@ -527,12 +539,34 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
   p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
   if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (grouped && layout) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
-  if (npes == 1 && !grouped && grid == sms) {
-    const int tiles = (a->M / BM) * (a->N / BN), kblocks = a->K / BK;
-    const SplitPlan plan = plan_split(tiles, kblocks, 2.0 * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N), sms);
-    // The persistent kernel: 6 us for launch, first loads and epilogue, then 0.29 us (pairs) or 0.36 us per K step and wave.
-    const double here = 6.0 + (double)((tiles + sms - 1) / sms) * kblocks * (pair ? 0.29 : 0.36);
-    if (plan.n_tile && plan.us < 0.97 * here) return launch_split(a, layout, 0, tiles, plan.n_tile, plan.splits, p.wait_limit_ns, stream);
+  // Time of the persistent kernel per K step and wave (us): 0.36 for single CTAs, 0.29 for pairs.
+  const int tmr = rows_per_pe / BM, tiles_n = a->N / BN, kblocks = a->K / BK;
+  SplitPlan tail = {0, 0, 0.0};
+  if (npes == 1 && !grouped) {
+    auto waves = [&](int blocks) { return (blocks * tiles_n + grid - 1) / grid; };
+    // One PE: an odd number of row blocks is rounded up for pairs where that costs less than single CTAs do (8320 x 8192 x 1024:
+    // 109 -> 98 us, 4224 x 3584 x 2048: 53.5 -> 48.3); not within one wave, where the pair's later start costs more
+    // (1152 x 2816 x 1984: 17 us single, 18.4 pairs).
+    const int even = (tmr + 1) & ~1;
+    if (pair_wanted() && grid >= 2 && !pair && waves(tmr) > 1) pair = waves(even) * 0.29 < waves(tmr) * 0.36;
+    p.row_blocks = pair ? even : tmr;
+    const double step = pair ? 0.29 : 0.36;
+    if (grid == sms) {
+      const double bytes = 2.0 * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N);
+      const SplitPlan plan = plan_split(tmr * tiles_n, kblocks, bytes, sms);
+      // 6 us for launch, first loads and the last epilogue
+      if (plan.n_tile && plan.us < 0.97 * (6.0 + waves(p.row_blocks) * kblocks * step))
+        return launch_split(a, layout, tmr, 0, tmr * tiles_n, false, plan, p.wait_limit_ns, stream);
+      // The last, partial wave: where its tiles, cut narrower and along K, take clearly less than a wave, they go to
+      // gemm_split_kernel, which starts on the SMs as this kernel leaves them.  4096 x 3584 x 8192 is 3.03 waves: 180 -> 166 us
+      // (power cap included); 8192 x 3584 x 4096, 6.05 waves: 173 -> 172.
+      const int total = p.row_blocks * tiles_n, per_wave = pair ? grid & ~1 : grid, rest = total % per_wave;
+      if (total > per_wave && rest) {
+        tail = plan_split(rest, kblocks, 0.0, sms);
+        if (tail.n_tile && tail.us < 0.85 * kblocks * step) p.tile_end = total - rest;
+        else tail.n_tile = 0;
+      }
+    }
   }
   int st = p.a_mn ? make_map(&p.tmA, a->A, a->K, a->M, BK) : make_map(&p.tmA, a->A, a->M, a->K, BM);
   if (st) return st;
@@ -629,7 +663,7 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
     return BSHMEM_FUSED_ERR_DRIVER;
   }
-  return 0;
+  return tail.n_tile ? launch_split(a, layout, p.row_blocks, p.tile_end, p.row_blocks * tiles_n - p.tile_end, true, tail, p.wait_limit_ns, stream) : 0;
 }
 
 extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stream) { return launch_gemm(a, 0, stream); }

@@ -51,6 +51,8 @@ struct alignas(64) FusedParams {
   const int* group_offsets;                  // GROUPED: device array [groups + 1], rows of group g are [offsets[g], offsets[g + 1])
   int groups, group_n;                       // GROUPED: number of groups; rows of B (output columns) per group
   int red_rows;                              // switch path: rows per work item of the reducing warps (16 or 32)
+  int row_blocks;                            // one PE: 128-row blocks that the tile order counts (pairs: rounded up to an even number; 0: as many as there are rows)
+  int tile_end;                              // one PE: tiles of the order that this kernel computes (0: all); gemm_split_kernel follows for the rest
   int a_mn, b_mn;                            // operand is stored with K outermost ([K][M] / [K][N]): loaded as it lies, no transpose pass
   int sw_reduce;                             // RS/AR: partial tiles stay local and the owner fetches their sum through the switch
 };
@@ -74,7 +76,7 @@ __host__ __device__ __forceinline__ TileInfo tile_info(const FusedParams& p, int
   TileInfo ti = tile_info_base(p, t);
   ti.a_row = ti.m_tile * BM;
   ti.b_row = ti.n_tile * BN;
-  ti.valid_rows = BM;
+  ti.valid_rows = ti.a_row < p.M ? BM : 0;  // 0: the block that an odd number of blocks was rounded up with
   return ti;
 }
 // GROUPED mode (C rows of group g = A rows of group g times B_g^T, group boundaries in device memory): `prefix[g]` is
@@ -104,7 +106,7 @@ __device__ __forceinline__ TileInfo grouped_tile_info(const FusedParams& p, cons
 }
 __host__ __device__ __forceinline__ TileInfo tile_info_base(const FusedParams& p, int t) {
   const int tiles_n = p.N / BN;
-  const int tmr = (p.M / p.npes) / BM;
+  const int tmr = p.row_blocks ? p.row_blocks : (p.M / p.npes) / BM;
   const int per_peer = tmr * tiles_n;
   TileInfo ti;
   if (p.sw_reduce) {
@@ -287,8 +289,17 @@ static inline int make_map(CUtensorMap* out, const void* base, uint64_t rows, ui
   cuuint64_t strides[1] = {cols * 2};
   cuuint32_t box[2] = {64, box_rows};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r != CUDA_SUCCESS) {
+    // A thread whose first CUDA call is this one (an autograd worker, say) has no current context yet: runtime calls would
+    // bind the device's own, a driver call does not.
+    int device = 0;
+    if (cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) r = encode();
+  }
   return r == CUDA_SUCCESS ? 0 : BSHMEM_FUSED_ERR_DRIVER;
 }
 

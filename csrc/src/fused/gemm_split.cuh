@@ -24,6 +24,8 @@ struct alignas(64) SplitParams {
   uint64_t wait_limit_ns;
   int M, N, K, act, a_mn, b_mn;
   int first_tile;  // in the order of the persistent kernel: 128 x 256 tiles, m fastest
+  int row_blocks;  // 128-row blocks of that order; the last may lie past M
+  int follows;     // the persistent kernel of the same product runs before this one
   int splits;
 };
 
@@ -84,7 +86,14 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
   uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int SUB = BN / N_TILE;  // tiles of this kernel per 128 x 256 tile
+  const int u = (int)blockIdx.x / p.splits, t = p.first_tile + u / SUB;
+  const int row0 = t % p.row_blocks * BM, col0 = t / p.row_blocks * BN + u % SUB * N_TILE;
   const int splits = p.splits, rank = (int)blockIdx.x % splits;
+  if (row0 >= p.M) {  // the whole cluster has no rows
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (int i = 0; i < STAGES; ++i) {
@@ -104,11 +113,10 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   // The launch may overlap the end of the kernel before it in the stream: nothing that it writes is touched before this.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // After the persistent kernel of the same product there is nothing to wait for (that one started when its inputs were
+  // complete, and writes other tiles) until the end, so that the end of this kernel is the end of both.
+  if (!p.follows) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  constexpr int SUB = BN / N_TILE;  // tiles of this kernel per 128 x 256 tile
-  const int u = (int)blockIdx.x / splits, t = p.first_tile + u / SUB, tiles_m = p.M / BM;
-  const int row0 = t % tiles_m * BM, col0 = t / tiles_m * BN + u % SUB * N_TILE;
   const int kblocks = p.K / BK, kb0 = kblocks * rank / splits, kb1 = kblocks * (rank + 1) / splits;
 
   if (warp == 0) {
@@ -186,6 +194,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const __gr
   else if (splits == 4) split_reduce_store<N_TILE, 4>(p, part, rank, row0, col0);
   else split_reduce_store<N_TILE, 8>(p, part, rank, row0, col0);
   if (splits > 1) cluster_sync_all();  // the peers have read my partial tile
+  if (p.follows) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (threadIdx.x == 0 && *abort_flag) atomicOr(p.error_flag, 1);
 }
 

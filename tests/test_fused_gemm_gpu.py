@@ -140,3 +140,49 @@ def test_products_of_few_tiles(M, N, K, act):
         fg.check_errors()
         assert bool(((got.double() - want).abs() <= want.abs() * 2 ** -8 + room).all()), (x_t, w_t)
     assert torch.equal(fg.gemm(x, w, act=act), fg.gemm(x, w, act=act))
+
+
+@pytest.mark.parametrize("M,N,K,act", [(2176, 2304, 192, None), (4480, 3584, 128, "gelu_tanh"), (2048, 4864, 1024, None), (3328, 3072, 2048, None), (1152, 8448, 64, None)])
+def test_odd_row_blocks_in_pairs_and_a_last_wave_cut_finer(M, N, K, act):
+    """More than a wave of tiles: an odd number of row blocks rounded up to pairs (the added block is neither loaded nor
+    stored), and the tiles of the last, partial wave on the kernel for few tiles; every element against float64."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    want = x.double() @ w.double().t()
+    room = 1e-4 * want.abs().max()  # order of the fp32 sums, as above
+    if act:
+        room = room + want.abs() * 2 ** -11
+        want = torch.nn.functional.gelu(want, approximate="tanh")
+    guard = torch.full((M + 128, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    for x_t, w_t in ((False, False), (True, True)):
+        got = fg.gemm(x.t().contiguous() if x_t else x, w.t().contiguous() if w_t else w, out=guard[:M], act=act, x_t=x_t, w_t=w_t)
+        torch.cuda.synchronize()
+        fg.check_errors()
+        assert bool(((got.double() - want).abs() <= want.abs() * 2 ** -8 + room).all()), (x_t, w_t)
+        assert bool((guard[M:] == 7.0).all()), "rows past the output were written"
+
+
+def test_gemm_is_a_threads_first_cuda_call():
+    """A thread that has not touched the GPU before (as an autograd worker may not have) calls the GEMM first."""
+    import threading
+    from nvshmem_b200.ops import fused_gemm as fg
+    x = torch.randn(128, 64, device="cuda").to(torch.bfloat16)
+    w = torch.randn(256, 64, device="cuda").to(torch.bfloat16)
+    want = fg.gemm(x, w)
+    out = torch.empty_like(want)
+    torch.cuda.synchronize()
+    failed = []
+
+    def work():
+        try:
+            fg.gemm(x, w, out=out)
+        except Exception as e:  # noqa: BLE001 - handed to the main thread
+            failed.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert not failed and torch.equal(out, want)
