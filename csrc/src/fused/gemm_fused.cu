@@ -42,6 +42,7 @@
 #include <mutex>
 
 #include "gemm_fused_common.cuh"
+#include "gemm_grouped.cuh"
 #include "gemm_split.cuh"
 
 namespace bshmem {
@@ -76,7 +77,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
   uint64_t* acc_empty = acc_full + 2;       // [2]
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-  int* g_prefix = (int*)(smem + SMEM_TILES + 256);  // GROUPED: [groups + 1] tiles before each group
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta_rank = PAIR ? cluster_ctarank() : 0;
@@ -100,17 +100,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
     tmem_alloc<PAIR ? 2 : 1>(tmem_slot, TMEM_COLS);
     tmem_relinquish<PAIR ? 2 : 1>();
   }
-  const bool grouped = p.mode == BSHMEM_FUSED_GROUPED;
-  if (grouped && warp == 3 && lane == 0) {
-    // Tiles per group from the group boundaries in device memory: no host round trip decides the work list.
-    int acc = 0;
-    for (int g = 0; g < p.groups; ++g) {
-      g_prefix[g] = acc;
-      const int rows = p.group_offsets[g + 1] - p.group_offsets[g];
-      acc += ((rows > 0 ? rows : 0) + BM - 1) / BM * (p.group_n / BN);
-    }
-    g_prefix[p.groups] = acc;
-  }
   tc_fence_before_sync();
   __syncthreads();
   if (PAIR) cluster_sync_all();  // the peer's barriers are initialised before anything arrives on them
@@ -118,7 +107,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_n = p.N / BN;
-  const int total_tiles = grouped ? g_prefix[p.groups] : p.tile_end ? p.tile_end : (p.row_blocks ? p.row_blocks : p.M / BM) * tiles_n;
+  const int total_tiles = p.tile_end ? p.tile_end : (p.row_blocks ? p.row_blocks : p.M / BM) * tiles_n;
   // The kernel for the last tiles needs nothing from this one: its CTAs may take the SMs as they become free.
   if (p.tile_end) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int kblocks = p.K / BK;
@@ -136,7 +125,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
       int stage = 0;
       uint32_t phase = 0;
       for (int t = first; t < total_tiles && !*abort_flag; t += step) {
-        const TileInfo ti = grouped ? grouped_tile_info(p, g_prefix, t) : tile_info(p, t);
+        const TileInfo ti = tile_info(p, t);
         if (p.mode == BSHMEM_FUSED_AG && ti.peer != p.rank) {
           // The 128 rows of this tile arrive from `peer`; all of K comes with them.
           // In-kernel sender: a counter per 128-row block.  External sender: one flag per shard, set to the call number.
@@ -233,7 +222,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
     uint32_t acc_phase = 0, chunk_counter = 0;
     uint64_t* pending_flag = nullptr;  // flag of the previous remote tile, published once its stores have completed
     for (int t = first; t < total_tiles; t += step) {
-      const TileInfo ti = grouped ? grouped_tile_info(p, g_prefix, t) : tile_info(p, t);
+      const TileInfo ti = tile_info(p, t);
       const bool own = !reduce_mode || (!sw && ti.peer == p.rank);
       uint32_t ok = mbar_wait(&acc_full[acc], acc_phase, p.wait_limit_ns, abort_flag) ? 1u : 0u;
       if (issuer && pending_flag) {
@@ -305,31 +294,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
             add8(v0);
             if (two) add8(v1);
           }
-        }
-        if (grouped) {
-          // Ragged tiles: every thread writes its own row straight from registers (128 contiguous bytes per chunk),
-          // rows past the end of the group are dropped.  No shared-memory staging, no bulk store.
-          if (p.act == BSHMEM_FUSED_ACT_SWIGLU) {
-            // Gated activation: the 64 columns of a chunk are 32 gate columns followed by their 32 up columns (the
-            // caller interleaves the weight rows that way); the output has half as many columns.
-#pragma unroll
-            for (int j = 0; j < EPI_COLS / 2; ++j) f[j] = f[j] / (1.0f + __expf(-f[j])) * f[EPI_COLS / 2 + j];
-          }
-          const int out_cols = p.act == BSHMEM_FUSED_ACT_SWIGLU ? EPI_COLS / 2 : EPI_COLS;
-          const size_t pitch = p.act == BSHMEM_FUSED_ACT_SWIGLU ? (size_t)p.group_n / 2 : (size_t)p.group_n;
-          if (row < ti.valid_rows) {
-            uint4* o = (uint4*)(p.out_local + ((size_t)(ti.a_row + row) * pitch + ((size_t)ti.n_tile * (BN / EPI_COLS) + (size_t)c) * out_cols) * 2);
-#pragma unroll
-            for (int j = 0; j < EPI_COLS / 8; ++j) {
-              if (j * 8 >= out_cols) break;
-              uint4 v;
-              __nv_bfloat162* h = (__nv_bfloat162*)&v;
-#pragma unroll
-              for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[j * 8 + 2 * e], f[j * 8 + 2 * e + 1]);
-              o[j] = v;
-            }
-          }
-          continue;
         }
         // Staging buffer (chunk_counter & 1) must have been drained by the TMA store issued two chunks ago.
         uint8_t* buf = sE + (chunk_counter & 1) * EPI_BUF;
@@ -414,8 +378,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
   if (threadIdx.x == 0 && *abort_flag) atomicOr(p.error_flag, 1);
 }
 
-static int g_attr_set_for_device = -1;
-
 // CTA pairs are the default where the shape allows them; BSHMEM_FUSED_2CTA=0 selects one CTA per tile.
 static bool pair_wanted() {
   static const bool on = [] {
@@ -453,6 +415,58 @@ static SplitPlan plan_split(int tiles, int kblocks, double bytes, int sms) {
 }
 
 // Tiles [first, first + tiles) of the product by gemm_split_kernel.
+// Raises a kernel's shared-memory limit, once per GPU (`ready`: the GPUs done, bit = ordinal).
+static bool reserve_smem(const void* kernel, int bytes, std::atomic<uint64_t>& ready) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return false;
+  if (device < 64 && (ready.load(std::memory_order_acquire) >> device & 1)) return true;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) {
+    fprintf(stderr, "bshmem_fused_gemm: cannot reserve %d bytes of shared memory: %s\n", bytes, cudaGetErrorString(e));
+    return false;
+  }
+  if (device < 64) ready.fetch_or(1ull << device, std::memory_order_release);
+  return true;
+}
+
+// GROUPED: pairs wherever two CTAs may run (the single-CTA build serves max_ctas = 1 and BSHMEM_FUSED_2CTA=0).
+static int launch_grouped(const bshmem_fused_args_t* a, int grid, uint64_t wait_limit_ns, cudaStream_t stream) {
+  GroupedParams p;
+  memset(&p, 0, sizeof(p));
+  if (((uintptr_t)a->out & 15)) return BSHMEM_FUSED_ERR_ALIGNMENT;
+  int st = make_map(&p.tmW, a->B, (uint64_t)a->groups * a->N, a->K, BM);
+  const bool pair = pair_wanted() && grid >= 2;
+  for (int i = 0; i < GRP_BOXES && !st; ++i) st = make_map(&p.tmX[i], a->A, a->M, a->K, GRP_STEP_N / (pair ? 2 : 1) * (i + 1));
+  if (st) return st;
+  p.out = (char*)a->out;
+  p.offsets = a->group_offsets;
+  p.error_flag = a->error_flag;
+  p.wait_limit_ns = wait_limit_ns;
+  p.groups = a->groups; p.N = a->N; p.K = a->K; p.act = a->act;
+  static void (*const kernels[4])(GroupedParams) = {gemm_grouped_kernel<false, false>, gemm_grouped_kernel<false, true>, gemm_grouped_kernel<true, false>, gemm_grouped_kernel<true, true>};
+  static std::atomic<uint64_t> ready[4];
+  const int which = (pair ? 2 : 0) + (a->act == BSHMEM_FUSED_ACT_SWIGLU ? 1 : 0);
+  if (!reserve_smem((const void*)kernels[which], GRP_SMEM, ready[which])) return BSHMEM_FUSED_ERR_DRIVER;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(pair ? grid & ~1 : grid);
+  cfg.blockDim = dim3(GRP_THREADS);
+  cfg.dynamicSmemBytes = GRP_SMEM;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pair ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], p);
+  if (e != cudaSuccess) {
+    fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
+    return BSHMEM_FUSED_ERR_DRIVER;
+  }
+  return 0;
+}
+
 // `row_blocks`: of the tile order (may be one more than there are rows for).  `follows`: the launch before it on the stream is
 // the persistent kernel of the same product.
 static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks, int first, int tiles, bool follows, SplitPlan plan, uint64_t wait_limit_ns,
@@ -477,15 +491,8 @@ static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks
   static void (*const kernels[6])(SplitParams) = {gemm_split_kernel<64, false>, gemm_split_kernel<64, true>, gemm_split_kernel<128, false>, gemm_split_kernel<128, true>,
                                                   gemm_split_kernel<256, false>, gemm_split_kernel<256, true>};
   const int which = (n_tile == 64 ? 0 : n_tile == 128 ? 2 : 4) + (layout ? 1 : 0);
-  static std::atomic<uint64_t> ready[6];  // per kernel: the GPUs (bit = ordinal) whose shared-memory limit is set
-  int device = 0;
-  cudaGetDevice(&device);
-  cudaError_t e = cudaSuccess;
-  if (device >= 64 || !(ready[which].load(std::memory_order_acquire) >> device & 1)) {
-    e = cudaFuncSetAttribute(kernels[which], cudaFuncAttributeMaxDynamicSharedMemorySize, SPLIT_SMEM);
-    if (e != cudaSuccess) return BSHMEM_FUSED_ERR_DRIVER;
-    if (device < 64) ready[which].fetch_or(1ull << device, std::memory_order_release);
-  }
+  static std::atomic<uint64_t> ready[6];
+  if (!reserve_smem((const void*)kernels[which], SPLIT_SMEM, ready[which])) return BSHMEM_FUSED_ERR_DRIVER;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles * (BN / n_tile) * splits);
   cfg.blockDim = dim3(SPLIT_THREADS);
@@ -500,7 +507,7 @@ static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = splits > 1 ? 2 : 1;
-  e = cudaLaunchKernelEx(&cfg, kernels[which], p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], p);
   if (e != cudaSuccess) {
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
     return BSHMEM_FUSED_ERR_DRIVER;
@@ -534,15 +541,15 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   int grid = a->max_ctas > 0 && a->max_ctas < sms ? a->max_ctas : sms;
   // A pair takes two consecutive 128-row tiles of one PE's block of rows.
-  bool pair = pair_wanted() && rows_per_pe % (2 * BM) == 0 && grid >= 2 && !grouped;  // ragged groups do not pair up
-  if (pair) grid &= ~1;
+  bool pair = pair_wanted() && rows_per_pe % (2 * BM) == 0 && grid >= 2;
   p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
   p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
-  if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (grouped && layout) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
+  if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
+  if (grouped) return launch_grouped(a, grid, p.wait_limit_ns, stream);
   // Time of the persistent kernel per K step and wave (us): 0.36 for single CTAs, 0.29 for pairs.
   const int tmr = rows_per_pe / BM, tiles_n = a->N / BN, kblocks = a->K / BK;
   SplitPlan tail = {0, 0, 0.0};
-  if (npes == 1 && !grouped) {
+  if (npes == 1) {
     auto waves = [&](int blocks) { return (blocks * tiles_n + grid - 1) / grid; };
     // One PE: an odd number of row blocks is rounded up for pairs where that costs less than single CTAs do (8320 x 8192 x 1024:
     // 109 -> 98 us, 4224 x 3584 x 2048: 53.5 -> 48.3); not within one wave, where the pair's later start costs more
@@ -625,27 +632,14 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
     }
     p.ag_external = a->ag_external != 0;
   }
-  if (grouped) {
-    if ((uintptr_t)a->out & 15) return BSHMEM_FUSED_ERR_ALIGNMENT;
-    p.group_offsets = a->group_offsets;
-    p.groups = a->groups;
-    p.group_n = a->N;
-    p.out_local = (char*)a->out;
-  }
   if (p.b_mn) st = make_map(&p.tmB, a->B, a->K, a->N, BK);
-  else st = make_map(&p.tmB, a->B, grouped ? (uint64_t)a->groups * a->N : (uint64_t)a->N, a->K, pair ? BN / 2 : BN);
+  else st = make_map(&p.tmB, a->B, a->N, a->K, pair ? BN / 2 : BN);
   if (st) return st;
   static void (*const kernels[4])(FusedParams) = {gemm_fused_kernel<false, false>, gemm_fused_kernel<false, true>, gemm_fused_kernel<true, false>, gemm_fused_kernel<true, true>};
-  if (g_attr_set_for_device != device) {
-    for (auto k : kernels) {
-      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-      if (e != cudaSuccess) {
-        fprintf(stderr, "bshmem_fused_gemm: cannot reserve %d bytes of shared memory: %s\n", SMEM_BYTES, cudaGetErrorString(e));
-        return BSHMEM_FUSED_ERR_DRIVER;
-      }
-    }
-    g_attr_set_for_device = device;
-  }
+  static std::atomic<uint64_t> ready[4];
+  const int which = (pair ? 2 : 0) + (layout ? 1 : 0);
+  if (!reserve_smem((const void*)kernels[which], SMEM_BYTES, ready[which])) return BSHMEM_FUSED_ERR_DRIVER;
+  if (pair) grid &= ~1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(NTHREADS);
@@ -658,7 +652,7 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pair ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[(pair ? 2 : 0) + (layout ? 1 : 0)], p);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], p);
   if (e != cudaSuccess) {
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
     return BSHMEM_FUSED_ERR_DRIVER;

@@ -186,3 +186,63 @@ def test_gemm_is_a_threads_first_cuda_call():
     t.join()
     torch.cuda.synchronize()
     assert not failed and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("sizes,N,K,act", [([1030, 0, 256, 257], 512, 320, None), ([1, 0, 0, 33], 256, 64, "gelu_tanh"), ([512, 513, 31, 225], 768, 128, "swiglu"),
+                                           ([0, 0, 0, 0], 256, 64, None), ([15, 16, 17, 32], 1024, 1088, "swiglu"), ([300] * 40, 256, 128, None)])
+def test_grouped_gemm_chunk_edges(sizes, N, K, act):
+    """Row counts at the edges of the 32-row steps and 256-row chunks, empty groups at either end, more groups than one
+    warp scans at once, every fused activation; rows outside the groups stay as they were."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(sum(sizes) + N + K)
+    G, first = len(sizes), 5                       # the first group does not start at row 0
+    offs = torch.zeros(G + 1, dtype=torch.int32)
+    offs[1:] = torch.tensor(sizes).cumsum(0).to(torch.int32)
+    offs += first
+    cap = int(offs[-1]) + 3
+    x = torch.randn(cap, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(G, N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    out_cols = N // 2 if act == "swiglu" else N
+    out = torch.full((cap, out_cols), 7.0, dtype=torch.bfloat16, device="cuda")
+    fg.grouped_gemm(x, fg.interleave_gate_up(w) if act == "swiglu" else w, offs.cuda(), out=out, act=act)
+    torch.cuda.synchronize()
+    fg.check_errors()
+    assert bool((out[:first] == 7.0).all()) and bool((out[int(offs[-1]):] == 7.0).all())
+    for g in range(G):
+        lo, hi = int(offs[g]), int(offs[g + 1])
+        if hi == lo:
+            continue
+        ref = x[lo:hi].double() @ w[g].double().t()
+        room = 1e-4 * ref.abs().max()              # order of the fp32 sums
+        if act == "swiglu":
+            # silu' is at most 1.1: the room of the gate, times the largest up value, and the other way round
+            room = 2.2 * room * ref.abs().max()
+            ref = torch.nn.functional.silu(ref[:, :N // 2]) * ref[:, N // 2:]
+        elif act:
+            room = room + ref.abs() * 2 ** -11     # the hardware tanh
+            ref = torch.nn.functional.gelu(ref, approximate="tanh")
+        assert bool(((out[lo:hi].double() - ref).abs() <= ref.abs() * 2 ** -8 + room).all()), (g, lo, hi)
+
+
+def test_grouped_gemm_on_one_cta_and_an_odd_number():
+    """`max_ctas` below two leaves no CTA pair; an odd limit leaves one CTA out.  Same values either way."""
+    import ctypes as C
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(3)
+    x = torch.randn(600, 128, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(3, 512, 128, device="cuda") * 0.05).to(torch.bfloat16)
+    offs = torch.tensor([0, 290, 291, 600], dtype=torch.int32, device="cuda")
+    want = fg.grouped_gemm(x, w, offs)
+    for limit in (1, 3):
+        out = torch.zeros_like(want)
+        a = fg._Args()
+        a.A, a.B, a.out = x.data_ptr(), w.data_ptr(), out.data_ptr()
+        a.M, a.N, a.K, a.npes, a.mode, a.epoch, a.max_ctas = 600, 512, 128, 1, fg.MODES["grouped"], 1, limit
+        a.group_offsets, a.groups, a.error_flag = offs.data_ptr(), 3, fg._error_flag(x.device).data_ptr()
+        assert fg.fused_lib().bshmem_fused_gemm(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        torch.cuda.synchronize()
+        fg.check_errors()
+        assert torch.equal(out, want)
+    big = torch.randn(1152, 64, device="cuda").to(torch.bfloat16)     # nine row blocks, odd limits for the plain product as well
+    wb = torch.randn(512, 64, device="cuda").to(torch.bfloat16)
+    assert torch.equal(fg.gemm(big, wb, max_ctas=5), fg.gemm(big, wb, max_ctas=1))
