@@ -230,6 +230,64 @@ def test_local_combine_over_column_ranges(nv, T, H, K):
     moe.close()
 
 
+@pytest.mark.parametrize("T,payload", [(40, "bf16"), (1200, "bf16"), (1200, "fp8")])
+def test_captured_calls_replay_on_new_inputs(nv, T, payload):
+    """Dispatch (one and two kernels), grouped GEMM, combine, a small GEMM, one with a finer last wave and a collective in one
+    CUDA graph, among them launches that overlap the kernel before: replays on new inputs equal eager calls."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    from nvshmem_b200.ops.moe import MoeDispatchCombine
+    torch.manual_seed(T)
+    H, K, E = 512, 4, 8
+    moe = MoeDispatchCombine(T, H, K, E, payload=payload)
+    w = (torch.randn(E, H, H, device="cuda") * 0.05).to(torch.bfloat16)
+    big_w = (torch.randn(2304, H, device="cuda") * 0.05).to(torch.bfloat16)
+    src, dst = nv.tensor((20011,), torch.float32), nv.tensor((20011,), torch.float32)
+    x, big = torch.empty(T, H, dtype=torch.bfloat16, device="cuda"), torch.empty(2176, H, dtype=torch.bfloat16, device="cuda")
+    idx, wt = torch.empty(T, K, dtype=torch.int32, device="cuda"), torch.empty(T, K, device="cuda")
+
+    def fill(seed):
+        torch.manual_seed(seed)
+        x.copy_(torch.randn(T, H, device="cuda"))
+        big.copy_(torch.randn(2176, H, device="cuda"))
+        idx.copy_(torch.rand(T, E, device="cuda").topk(K).indices)
+        wt.copy_(torch.rand(T, K, device="cuda"))
+        src.copy_(torch.randn(20011, device="cuda"))
+
+    def calls():
+        recv, offs = moe.dispatch(x, idx)
+        if payload == "bf16":
+            fg.grouped_gemm(recv, w, offs, out=moe.expert_out)
+        else:
+            moe.expert_out.copy_(moe.dequantized(moe.cap_rows))
+        y = fg.gemm(fg.gemm(big, big_w)[:256, :H].contiguous(), big_w[:256])
+        nv.reduce(0, dst, src, "sum")
+        return moe.combine(idx, wt), y, dst
+
+    fill(1)
+    calls()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = calls()
+    torch.cuda.synchronize()
+    for seed in (2, 3):
+        fill(seed)
+        want = [t.clone() for t in calls()]
+        for t in out:
+            t.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        fg.check_errors()
+        for got, ref in zip(out, want):
+            assert torch.equal(got, ref)
+    moe.close()
+    nv.free_tensor(src)
+    nv.free_tensor(dst)
+
+
 @pytest.mark.parametrize("payload,tol", [("bf16", 0.03), ("fp8", 0.08)])
 def test_moe_block_matches_fp32_reference_single_pe(nv, payload, tol):
     """Router + dispatch + expert MLPs + combine against a plain PyTorch fp32 version of the same block."""
