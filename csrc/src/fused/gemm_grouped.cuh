@@ -63,7 +63,7 @@ __device__ __forceinline__ GroupTile group_tile(const GroupedParams& p, const in
     if (prefix[mid] <= t) lo = mid;
     else hi = mid;
   }
-  const int local = t - prefix[lo], r0 = p.offsets[lo], total = p.offsets[lo + 1] - r0;
+  const int local = t - prefix[lo], r0 = __ldcg(p.offsets + lo), total = __ldcg(p.offsets + lo + 1) - r0;
   // chunks run fastest: CTAs that run together share the weights through L2
   const int chunks = group_chunks(total), n = group_chunk_rows(total);
   const int c = local % chunks;
@@ -110,11 +110,15 @@ __global__ void __launch_bounds__(GRP_THREADS, 1) gemm_grouped_kernel(const __gr
     tmem_alloc<PAIR ? 2 : 1>(tmem_slot, TMEM_COLS);
     tmem_relinquish<PAIR ? 2 : 1>();
   }
+  // The launch may overlap the end of the kernel before it on the stream: what that one writes (the boundaries among it) is
+  // read only after this.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp == 3) {
     int tiles = 0, max_n = GRP_STEP_N;
     for (int base = 0; base < p.groups; base += 32) {
       const int g = base + lane;
-      const int rows = g < p.groups ? max(0, p.offsets[g + 1] - p.offsets[g]) : 0;
+      const int rows = g < p.groups ? max(0, __ldcg(p.offsets + g + 1) - __ldcg(p.offsets + g)) : 0;
       const int mine = group_chunks(rows) * (p.N / W_ROWS);
       int upto = mine;
 #pragma unroll
