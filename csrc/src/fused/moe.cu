@@ -625,8 +625,19 @@ __global__ void __cluster_dims__(ROUTE_CTAS, 1, 1) __launch_bounds__(ROUTE_THREA
   __syncthreads();
   const long pairs = (long)a.T * a.K, per = (pairs + ROUTE_CTAS - 1) / ROUTE_CTAS;
   const long lo = min(pairs, per * me), hi = min(pairs, per * (me + 1));
+  // The first ROUTE_HELD pairs of a thread stay in registers (all of a batch of 8192 tokens x 8), the rest goes by way of slot_map.
+  constexpr int ROUTE_HELD = 8;
+  int held_e[ROUTE_HELD], held_pos[ROUTE_HELD];
+#pragma unroll
+  for (int h = 0; h < ROUTE_HELD; ++h) {
+    const long i = lo + threadIdx.x + (long)h * ROUTE_THREADS;
+    held_e[h] = i < hi ? a.topk_idx[i] : -1;
+  }
+#pragma unroll
+  for (int h = 0; h < ROUTE_HELD; ++h) held_pos[h] = held_e[h] >= 0 && held_e[h] < E ? atomicAdd(&s_count[held_e[h]], 1) : -1;
+  const long rest = lo + threadIdx.x + (long)ROUTE_HELD * ROUTE_THREADS;
 #pragma unroll 4
-  for (long i = lo + threadIdx.x; i < hi; i += ROUTE_THREADS) {
+  for (long i = rest; i < hi; i += ROUTE_THREADS) {
     const int e = a.topk_idx[i];
     a.slot_map[i] = e >= 0 && e < E ? atomicAdd(&s_count[e], 1) : -1;
   }
@@ -647,8 +658,13 @@ __global__ void __cluster_dims__(ROUTE_CTAS, 1, 1) __launch_bounds__(ROUTE_THREA
   cluster.sync();  // nobody reads the counts, or the starts, any more
   if ((int)threadIdx.x < E) s_start[threadIdx.x] += before;
   __syncthreads();
+#pragma unroll
+  for (int h = 0; h < ROUTE_HELD; ++h) {
+    const long i = lo + threadIdx.x + (long)h * ROUTE_THREADS;
+    if (i < hi) a.slot_map[i] = held_pos[h] >= 0 ? local_row(a, s_start[held_e[h]] + held_pos[h]) : -1;
+  }
 #pragma unroll 4
-  for (long i = lo + threadIdx.x; i < hi; i += ROUTE_THREADS) {
+  for (long i = rest; i < hi; i += ROUTE_THREADS) {
     const int e = a.topk_idx[i];
     if (e >= 0 && e < E) a.slot_map[i] = local_row(a, s_start[e] + a.slot_map[i]);
   }

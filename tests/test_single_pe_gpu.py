@@ -156,7 +156,7 @@ def test_moe_dispatch_combine_single_pe(nv):
 
 @pytest.mark.parametrize("payload", [0, 1])
 @pytest.mark.parametrize("T,H,K,E,cap", [(1, 128, 1, 1, 0), (3, 640, 16, 1024, 0), (128, 256, 16, 64, 0), (2049, 128, 1, 7, 0), (683, 2176, 3, 5, 0),
-                                         (700, 2304, 8, 256, 0), (9000, 384, 9, 1000, 0), (100, 256, 4, 8, 77), (1000, 1152, 8, 8, 5000), (5, 16512, 2, 4, 0)])
+                                         (700, 2304, 8, 256, 0), (9000, 384, 9, 1000, 0), (8193, 128, 8, 33, 0), (100, 256, 4, 8, 77), (1000, 1152, 8, 8, 5000), (5, 16512, 2, 4, 0)])
 def test_local_dispatch_agrees_with_the_general_one(T, H, K, E, cap, payload):
     """One PE without `dup_src` takes the kernels that meet nobody (one for up to 2048 pairs, two above); with `dup_src` the
     general kernel runs.  Offsets, counts and the multiset of rows per expert must be the same, and every row must hold what its slot
