@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(GRP_THREADS, 1) gemm_grouped_kernel(const __gr
     const int team = (warp - EPI_WARP0) >> 2, ew = warp & 3, et = (int)threadIdx.x & (EPI_THREADS - 1);
     constexpr int OUT_COLS = GATED ? BM / 2 : BM, PER_ROW = OUT_COLS / 8;  // output columns of this CTA's half of a tile; 16-byte pieces of a row
     uint8_t* mine = staging + team * GRP_STAGING;           // two buffers [32 rows][OUT_COLS] bf16
-    float* ex = (float*)(mine + 8192) + (ew >> 1) * 1024;   // gated: [32 rows][32 columns] fp32 from the up warp to its gate warp
+    float* ex = (float*)(mine + 8192) + (ew >> 1) * 1024;   // gated: [32 rows][32 columns] fp32 between a gate warp and its up warp
     const size_t pitch = GATED ? (size_t)p.N / 2 : (size_t)p.N;
     int acc = 0, buf = 0;
     uint32_t acc_phase = 0;
@@ -245,14 +245,25 @@ __global__ void __launch_bounds__(GRP_THREADS, 1) gemm_grouped_kernel(const __gr
         __nv_bfloat16* tile = (__nv_bfloat16*)(mine + buf * (32 * OUT_COLS * 2));
         if (GATED) {
           // The weight rows are 32 gate rows followed by their 32 up rows: warps 0 and 2 hold gates, 1 and 3 the matching ups.
+          // The gate warp finishes the first 16 rows and the up warp the others; each hands over what the other one needs.
           if (ew & 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) ex[j * 32 + lane] = f[j];
+            for (int j = 0; j < 16; ++j) ex[j * 32 + lane] = f[j];
+          } else {
+#pragma unroll
+            for (int j = 16; j < 32; ++j) ex[j * 32 + lane] = f[j];
           }
           named_bar_sync(1 + GRP_EPI + team * 2 + (ew >> 1), 64);
-          if (!(ew & 1)) {
+          __nv_bfloat16* to = tile + (ew >> 1) * 32 + lane;
+          if (ew & 1) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) tile[j * OUT_COLS + (ew >> 1) * 32 + lane] = __float2bfloat16_rn(f[j] / (1.0f + __expf(-f[j])) * ex[j * 32 + lane]);
+            for (int j = 16; j < 32; ++j) {
+              const float gate = ex[j * 32 + lane];
+              to[j * OUT_COLS] = __float2bfloat16_rn(gate / (1.0f + __expf(-gate)) * f[j]);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) to[j * OUT_COLS] = __float2bfloat16_rn(f[j] / (1.0f + __expf(-f[j])) * ex[j * 32 + lane]);
           }
         } else {
 #pragma unroll

@@ -1,5 +1,5 @@
 // Expert-parallel MoE dispatch and combine for sm_100a over NVLink peer memory.  What follows is the form for several PEs; one
-// PE has kernels without any barrier (see "dispatch on one PE" and combine_kernel<KT, true>).
+// PE has kernels without any barrier (see "dispatch on one PE" and combine_kernel with LOCAL).
 //
 // dispatch (one cooperative kernel, persistent CTAs of 256 threads):
 //   A  histogram of the K expert ids of every token (shared-memory bins, then global atomics)
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(THREADS) dispatch_kernel(const __grid_constant
 // Weighted sum of up to KT expert rows into one output row.  Row pointers and weights sit in registers;
 // for every 16-byte column block the KT loads are issued before the first is consumed.
 template <int KT>
-__device__ __forceinline__ void combine_token(const uint8_t* const* src, const float* wt, int K, uint4* out_row, int c_first, int c_end) {
+__device__ __forceinline__ void combine_token(const uint8_t* const* src, const float* wt, int K, uint4* out_row, int c_first, int c_end, const int c_step) {
   const uint4* p[KT];
   float w[KT];
 #pragma unroll
@@ -370,7 +370,7 @@ __device__ __forceinline__ void combine_token(const uint8_t* const* src, const f
     p[j] = on ? (const uint4*)src[j] : nullptr;
     w[j] = on ? wt[j] : 0.f;
   }
-  for (int c = c_first + threadIdx.x; c < c_end; c += THREADS) {
+  for (int c = c_first; c < c_end; c += c_step) {
     uint4 v[KT];
 #pragma unroll
     for (int j = 0; j < KT; ++j) v[j] = p[j] ? p[j][c] : make_uint4(0u, 0u, 0u, 0u);
@@ -395,9 +395,12 @@ __device__ __forceinline__ void combine_token(const uint8_t* const* src, const f
 
 // LOCAL (one PE): nobody to meet on entry or exit, so no barrier, no cooperative launch and no cleared counter; the work items
 // are `split` column ranges of every token, so that a decode batch of few tokens still fills the SMs.  Bound by HBM reads.
-// H 7168, top-8: 4096 tokens 88 -> 82 us (6.4 TB/s), 64 tokens 13 -> 6.7 us.
-template <int KT, bool LOCAL>
-__global__ void __launch_bounds__(THREADS, KT <= 8 ? 3 : 2) combine_kernel(const __grid_constant__ CombineParams P) {
+// H 7168, top-8: 4096 tokens 88 -> 82 us (6.4 TB/s), 64 tokens 13 -> 6.7 us;
+// H 128, top-4, 16364 tokens: 36.6 -> 6.7 us.
+// NARROW: rows (or column ranges) of at most half as many 16-byte pieces as the CTA has threads are taken several at a time,
+// a power of two of threads each; a build of its own because the variable stride costs wide rows 3 %.
+template <int KT, bool LOCAL, bool NARROW>
+__global__ void __launch_bounds__(THREADS, KT <= 8 ? 4 : 3) combine_kernel(const __grid_constant__ CombineParams P) {
   const bshmem_moe_combine_args_t& a = P.a;
   const int H = a.H, K = a.K, E = a.E, npes = a.npes, rank = a.rank;
   const int EL = E / npes;
@@ -412,6 +415,12 @@ __global__ void __launch_bounds__(THREADS, KT <= 8 ? 3 : 2) combine_kernel(const
     if (!grid_barrier(&sc->grid_bar, phase, P.wait_limit_ns, a.error_flag)) return;
   }
   const int per_chunk = THREADS / K;
+  int lanes = THREADS;
+  if (NARROW) {
+    const int per_item = (nvec + split - 1) / split;
+    lanes = 16;  // H is a multiple of 128: 16 pieces at least
+    while (lanes < per_item) lanes *= 2;
+  }
   for (int base = 0; (long)blockIdx.x + (long)base * gridDim.x < items; base += per_chunk) {
     __syncthreads();
     {
@@ -429,13 +438,13 @@ __global__ void __launch_bounds__(THREADS, KT <= 8 ? 3 : 2) combine_kernel(const
       }
     }
     __syncthreads();
-    for (int i = 0; i < per_chunk; ++i) {
+    for (int i = NARROW ? (int)threadIdx.x / lanes : 0; i < per_chunk; i += NARROW ? THREADS / lanes : 1) {
       const long it = (long)blockIdx.x + (long)(base + i) * gridDim.x;
       if (it >= items) break;
-      const long t = it / split;
+      const long t = split == 1 ? it : it / split;
       const int part = (int)(it - t * split);
       uint4* out_row = (uint4*)a.out + (size_t)t * nvec;
-      combine_token<KT>(s_src + i * K, s_w + i * K, K, out_row, (int)((long)nvec * part / split), (int)((long)nvec * (part + 1) / split));
+      combine_token<KT>(s_src + i * K, s_w + i * K, K, out_row, nvec * part / split + (NARROW ? (int)threadIdx.x % lanes : (int)threadIdx.x), nvec * (part + 1) / split, NARROW ? lanes : THREADS);
     }
   }
   if (LOCAL) return;
@@ -450,8 +459,8 @@ __global__ void __launch_bounds__(THREADS, KT <= 8 ? 3 : 2) combine_kernel(const
 //    L2) and finds the place of its own token's rows by counting the equal ids before them;
 //  * more: a routing kernel (one cluster of eight CTAs, counts met through distributed shared memory) writes the slot map and
 //    the offsets, then a kernel that only moves rows.
-// Device time, 64 tokens x 7168, top-8 of 256: 16.5 us before, 7 us now; 4096 tokens: bf16 112 us -> 8.5 (routing) + 91
-// (529 MB, 5.8 TB/s), fp8 79.6 us -> 9 + 51.5 (5.8 TB/s), bound by HBM writes.  The row kernel is launched early and loads
+// Device time, 64 tokens x 7168, top-8 of 256: 16.5 us before, 7 us now; 4096 tokens: bf16 112 us -> 6.3 (routing) + 91
+// (529 MB, 5.8 TB/s), fp8 79.6 us -> 6.5 + 51.5 (5.8 TB/s), bound by HBM writes.  The row kernel is launched early and loads
 // token rows while the routing runs (2.5 us less).
 constexpr int LOCAL_SMALL_PAIRS = 2048, ROUTE_CTAS = 8, ROUTE_THREADS = 1024;
 
@@ -903,16 +912,17 @@ extern "C" int bshmem_moe_combine(const bshmem_moe_combine_args_t* a, cudaStream
   P.split = 1;
   if (a->npes == 1) {
     P.split = column_split(a->T, a->H / BSHMEM_MOE_QUANT_BLOCK);
-    st = a->K <= 8 ? coop_grid(combine_kernel<8, true>, 0, a->T * P.split, a->max_ctas, &grid)
-                   : coop_grid(combine_kernel<BSHMEM_MOE_MAX_TOPK, true>, 0, a->T * P.split, a->max_ctas, &grid);
+    const bool narrow = (a->H / 8 + P.split - 1) / P.split <= THREADS / 2;
+    auto kernel = a->K <= 8 ? (narrow ? combine_kernel<8, true, true> : combine_kernel<8, true, false>)
+                            : (narrow ? combine_kernel<BSHMEM_MOE_MAX_TOPK, true, true> : combine_kernel<BSHMEM_MOE_MAX_TOPK, true, false>);
+    st = coop_grid(kernel, 0, a->T * P.split, a->max_ctas, &grid);
     if (st) return st;
-    if (a->K <= 8) combine_kernel<8, true><<<grid, THREADS, 0, stream>>>(P);
-    else combine_kernel<BSHMEM_MOE_MAX_TOPK, true><<<grid, THREADS, 0, stream>>>(P);
+    kernel<<<grid, THREADS, 0, stream>>>(P);
     return launched("bshmem_moe_combine", cudaGetLastError());
   }
   // Two builds of the kernel: up to 8 choices per token (fewer registers, three CTAs per SM) and up to 16.
-  const void* kernel = a->K <= 8 ? (const void*)combine_kernel<8, false> : (const void*)combine_kernel<BSHMEM_MOE_MAX_TOPK, false>;
-  st = a->K <= 8 ? coop_grid(combine_kernel<8, false>, 0, a->T, a->max_ctas, &grid) : coop_grid(combine_kernel<BSHMEM_MOE_MAX_TOPK, false>, 0, a->T, a->max_ctas, &grid);
+  const void* kernel = a->K <= 8 ? (const void*)combine_kernel<8, false, false> : (const void*)combine_kernel<BSHMEM_MOE_MAX_TOPK, false, false>;
+  st = a->K <= 8 ? coop_grid(combine_kernel<8, false, false>, 0, a->T, a->max_ctas, &grid) : coop_grid(combine_kernel<BSHMEM_MOE_MAX_TOPK, false, false>, 0, a->T, a->max_ctas, &grid);
   if (st) return st;
   if (cudaMemsetAsync(a->scratch, 0, 256, stream) != cudaSuccess) return BSHMEM_MOE_ERR_DRIVER;  // the grid-barrier counter
   void* params[] = {(void*)&P};

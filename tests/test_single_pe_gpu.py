@@ -210,7 +210,7 @@ def test_local_dispatch_agrees_with_the_general_one(T, H, K, E, cap, payload):
         assert torch.equal(local[0][rows].view(torch.bfloat16), x[t])
 
 
-@pytest.mark.parametrize("T,H,K", [(1, 128, 1), (3, 640, 16), (61, 7168, 8), (295, 256, 9), (1500, 384, 4)])
+@pytest.mark.parametrize("T,H,K", [(1, 128, 1), (3, 640, 16), (61, 7168, 8), (295, 256, 9), (1500, 384, 4), (5000, 128, 16), (4001, 2176, 1)])
 def test_local_combine_over_column_ranges(nv, T, H, K):
     """Few tokens: a token's row is cut into column ranges for several CTAs.  fp32 sums of K products, one rounding to bf16."""
     from nvshmem_b200.ops.moe import MoeDispatchCombine
