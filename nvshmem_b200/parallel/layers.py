@@ -93,7 +93,7 @@ class _RowParallelFn(torch.autograd.Function):
     def backward(ctx, dy_shard):
         x, weight = ctx.saved_tensors
         if dy_shard.shape[0] == ctx.M:  # one PE: the shard is the whole, nothing to gather
-            dy = _aligned(dy_shard)
+            dy = _aligned(dy_shard.to(torch.bfloat16))
             return fg.gemm(dy, _aligned(weight), w_t=True), fg.gemm(dy, _aligned(x), x_t=True, w_t=True), None
         # dX[M, Kl] = all_gather(dY_shard)[M, N] @ W[N, Kl]
         ag = ctx.cache.all_gather(ctx.M, ctx.N)
