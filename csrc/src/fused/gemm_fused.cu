@@ -27,7 +27,7 @@
 //            a flag write per shard; no SM takes part) or by the auxiliary warps of all CTAs (a counter per 128-row
 //            block); the producer warp consumes shards in arrival order (own, then rank-1, rank-2, …) and only waits
 //            when one has not landed.  Remote data is always read from this GPU's own memory.
-//   MODE_PLAIN  no collective (also what 1 PE runs; products of few tiles go to gemm_split_kernel, see gemm_split.cuh).
+//   MODE_PLAIN  no collective (also what 1 PE runs; products of few tiles go to gemm_narrow_kernel, see gemm_narrow.cuh).
 // Every wait (mbarrier, flag) is bounded; on expiry the CTA unwinds, frees its tensor memory and sets `error_flag`.
 // No load uses a cluster-wide broadcast form, so the same binary runs on any number of GPUs.
 // (reference for the capability: examples/gemm_allreduce/*, which fuses a CUTLASS GEMM with an NVLS allreduce)
@@ -43,7 +43,7 @@
 
 #include "gemm_fused_common.cuh"
 #include "gemm_grouped.cuh"
-#include "gemm_split.cuh"
+#include "gemm_narrow.cuh"
 
 namespace bshmem {
 using namespace sm100;
@@ -392,34 +392,31 @@ static bool pair_wanted() {
   return on;
 }
 
-// The tile width and the number of K parts for `tiles` output tiles of 128 x 256, if one wave of CTAs can hold them.  A model
-// of measured times (us): a fixed part (launch, first loads, reduction through the cluster, store) and, per 64-wide K step,
-// the time an SM needs to load a stage (about 70 bytes per clock whatever the tile), or that of all the bytes from HBM.
-//   128 x 512 x 512     64/1 4.6   64/4 5.3   128/1 5.5   256/1 7.7    (persistent kernel 8.0)
-//   128 x 1024 x 2048   64/1 7.8   64/4 6.2   128/4 7.4   256/4 10.4   (14.9)
-//   128 x 3584 x 8192   64/2 17.1  128/2 21.3  128/4 16.8  256/4 22.6  (52.0)
-//   512 x 3584 x 8192   128/1 31.8  256/2 32.7                         (43.4)
-// Clusters of eight find too few places when there are many (16 of them ran in two waves), clusters of four find 32.
-struct SplitPlan {
-  int n_tile, splits;
+// The tile width for `tiles` output tiles of 128 x 256, if one wave of CTAs can hold them: the one of least time by a model of
+// measured times, in us: a fixed part (launch, first loads, store) and, per 64-wide K step, what an SM takes to load a stage of cold
+// operands, or all the bytes from HBM.  Weights warm / cold in L2, rows of both: the width, the persistent kernel last.
+//   128 x 512 x 512     64 3.5 / 3.4     128 4.1 / 4.1     256 6.1 / 6.1     6.9 / 6.7
+//   128 x 3584 x 8192   64 19.0 / 22.8   128 21.6 / 30.7   256 39.5 / 50.6   40.4 / 50.9
+//   512 x 3584 x 8192                    128 25.3 / 30.7   256 39.6 / 50.3   41.6 / 43.0
+//   1152 x 2816 x 1984                                     256 14.0 / 15.6   14.8 / 16.3
+// So a step of cold operands takes 0.15 (24 KB), 0.21 (32 KB) and 0.36 us (48 KB), of warm ones 0.13, 0.15 and 0.28.
+struct NarrowPlan {
+  int n_tile;  // 0: none
   double us;
 };
-static SplitPlan plan_split(int tiles, int kblocks, double bytes, int sms) {
+static NarrowPlan plan_narrow(int tiles, int kblocks, double bytes, int sms) {
   static const int width[3] = {64, 128, 256};
-  static const double fixed[3][4] = {{2.6, 4.0, 4.1, 4.3}, {3.4, 5.3, 5.0, 5.4}, {4.5, 7.3, 7.0, 7.7}}, step[3] = {0.14, 0.20, 0.36};
-  SplitPlan best = {0, 0, 0.0};
-  for (int w = 0; w < 3; ++w)
-    for (int l = 0; l < 4; ++l) {
-      const int splits = 1 << l, most = l == 3 ? sms * 7 / 16 : l == 2 ? sms * 7 / 8 : sms;
-      if ((long)tiles * (BN / width[w]) * splits > most || splits > kblocks) continue;
-      const double loads = ((kblocks + splits - 1) / splits) * step[w], hbm = bytes / 6.2e6;
-      const double us = fixed[w][l] + (loads > hbm ? loads : hbm);
-      if (!best.n_tile || us < best.us) best = {width[w], splits, us};
-    }
+  static const double fixed[3] = {2.6, 3.4, 4.5}, step[3] = {0.14, 0.20, 0.36};
+  NarrowPlan best = {0, 0.0};
+  for (int w = 0; w < 3; ++w) {
+    if ((long)tiles * (BN / width[w]) > sms) continue;
+    const double loads = kblocks * step[w], hbm = bytes / 6.2e6;
+    const double us = fixed[w] + (loads > hbm ? loads : hbm);
+    if (!best.n_tile || us < best.us) best = {width[w], us};
+  }
   return best;
 }
 
-// Tiles [first, first + tiles) of the product by gemm_split_kernel.
 // Launch attributes: `overlap` lets the launch begin before the kernel before it on the stream has ended (the kernel waits
 // itself, griddepcontrol.wait; 1 to 1.5 us less between dependent kernels), `cluster` CTAs form a cluster.
 static int launch_attributes(cudaLaunchAttribute* attr, bool overlap, int cluster) {
@@ -485,12 +482,12 @@ static int launch_grouped(const bshmem_fused_args_t* a, int grid, uint64_t wait_
   return 0;
 }
 
-// `row_blocks`: of the tile order (may be one more than there are rows for).  `follows`: the launch before it on the stream is
-// the persistent kernel of the same product.
-static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks, int first, int tiles, bool follows, SplitPlan plan, uint64_t wait_limit_ns,
-                        cudaStream_t stream) {
-  const int n_tile = plan.n_tile, splits = plan.splits;
-  SplitParams p;
+// Tiles [first, first + tiles) of the product by gemm_narrow_kernel.  `row_blocks`: of the tile order (may be one more than there
+// are rows for).  `follows`: the launch before it on the stream is the persistent kernel of the same product.
+static int launch_narrow(const bshmem_fused_args_t* a, int layout, int row_blocks, int first, int tiles, bool follows, NarrowPlan plan, uint64_t wait_limit_ns,
+                         cudaStream_t stream) {
+  const int n_tile = plan.n_tile;
+  NarrowParams p;
   memset(&p, 0, sizeof(p));
   p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
   p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
@@ -505,20 +502,19 @@ static int launch_split(const bshmem_fused_args_t* a, int layout, int row_blocks
   p.first_tile = first;
   p.row_blocks = row_blocks;
   p.follows = follows;
-  p.splits = splits;
-  static void (*const kernels[6])(SplitParams) = {gemm_split_kernel<64, false>, gemm_split_kernel<64, true>, gemm_split_kernel<128, false>, gemm_split_kernel<128, true>,
-                                                  gemm_split_kernel<256, false>, gemm_split_kernel<256, true>};
+  static void (*const kernels[6])(NarrowParams) = {gemm_narrow_kernel<64, false>, gemm_narrow_kernel<64, true>, gemm_narrow_kernel<128, false>, gemm_narrow_kernel<128, true>,
+                                                   gemm_narrow_kernel<256, false>, gemm_narrow_kernel<256, true>};
   const int which = (n_tile == 64 ? 0 : n_tile == 128 ? 2 : 4) + (layout ? 1 : 0);
   static std::atomic<uint64_t> ready[6];
-  if (!reserve_smem((const void*)kernels[which], SPLIT_SMEM, ready[which])) return BSHMEM_FUSED_ERR_DRIVER;
+  if (!reserve_smem((const void*)kernels[which], NARROW_SMEM, ready[which])) return BSHMEM_FUSED_ERR_DRIVER;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(tiles * (BN / n_tile) * splits);
-  cfg.blockDim = dim3(SPLIT_THREADS);
-  cfg.dynamicSmemBytes = SPLIT_SMEM;
+  cfg.gridDim = dim3(tiles * (BN / n_tile));
+  cfg.blockDim = dim3(NARROW_THREADS);
+  cfg.dynamicSmemBytes = NARROW_SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];
   cfg.attrs = attr;
-  cfg.numAttrs = launch_attributes(attr, true, splits);
+  cfg.numAttrs = launch_attributes(attr, true, 1);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernels[which], p);
   if (e != cudaSuccess) {
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
@@ -560,7 +556,7 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   if (grouped) return launch_grouped(a, grid, p.wait_limit_ns, stream);
   // Time of the persistent kernel per K step and wave (us): 0.36 for single CTAs, 0.29 for pairs.
   const int tmr = rows_per_pe / BM, tiles_n = a->N / BN, kblocks = a->K / BK;
-  SplitPlan tail = {0, 0, 0.0};
+  NarrowPlan tail = {0, 0.0};
   if (npes == 1) {
     auto waves = [&](int blocks) { return (blocks * tiles_n + grid - 1) / grid; };
     // One PE: an odd number of row blocks is rounded up for pairs where that costs less than single CTAs do (8320 x 8192 x 1024:
@@ -572,16 +568,16 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
     const double step = pair ? 0.29 : 0.36;
     if (grid == sms) {
       const double bytes = 2.0 * ((double)a->M * a->K + (double)a->N * a->K + (double)a->M * a->N);
-      const SplitPlan plan = plan_split(tmr * tiles_n, kblocks, bytes, sms);
+      const NarrowPlan plan = plan_narrow(tmr * tiles_n, kblocks, bytes, sms);
       // 6 us for launch, first loads and the last epilogue
       if (plan.n_tile && plan.us < 0.97 * (6.0 + waves(p.row_blocks) * kblocks * step))
-        return launch_split(a, layout, tmr, 0, tmr * tiles_n, false, plan, p.wait_limit_ns, stream);
-      // The last, partial wave: where its tiles, cut narrower and along K, take clearly less than a wave, they go to
-      // gemm_split_kernel, which starts on the SMs as this kernel leaves them.  4096 x 3584 x 8192 is 3.03 waves: 180 -> 166 us
+        return launch_narrow(a, layout, tmr, 0, tmr * tiles_n, false, plan, p.wait_limit_ns, stream);
+      // The last, partial wave: where its tiles, cut narrower, take clearly less than a wave, they go to
+      // gemm_narrow_kernel, which starts on the SMs as this kernel leaves them.  4096 x 3584 x 8192 is 3.03 waves: 180 -> 168 us
       // (power cap included); 8192 x 3584 x 4096, 6.05 waves: 173 -> 172.
       const int total = p.row_blocks * tiles_n, per_wave = pair ? grid & ~1 : grid, rest = total % per_wave;
       if (total > per_wave && rest) {
-        tail = plan_split(rest, kblocks, 0.0, sms);
+        tail = plan_narrow(rest, kblocks, 0.0, sms);
         if (tail.n_tile && tail.us < 0.85 * kblocks * step) p.tile_end = total - rest;
         else tail.n_tile = 0;
       }
@@ -665,7 +661,7 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
     fprintf(stderr, "bshmem_fused_gemm: launch failed: %s\n", cudaGetErrorString(e));
     return BSHMEM_FUSED_ERR_DRIVER;
   }
-  return tail.n_tile ? launch_split(a, layout, p.row_blocks, p.tile_end, p.row_blocks * tiles_n - p.tile_end, true, tail, p.wait_limit_ns, stream) : 0;
+  return tail.n_tile ? launch_narrow(a, layout, p.row_blocks, p.tile_end, p.row_blocks * tiles_n - p.tile_end, true, tail, p.wait_limit_ns, stream) : 0;
 }
 
 extern "C" int bshmem_fused_gemm(const bshmem_fused_args_t* a, cudaStream_t stream) { return launch_gemm(a, 0, stream); }
@@ -683,12 +679,8 @@ extern "C" int bshmem_fused_test_ag_units(int K, int grid, int* out) {
   return 0;
 }
 
-// Test hook (host only): what plan_split chooses; out = {tile width (0: the persistent kernel), K parts}.
-extern "C" void bshmem_fused_test_split_plan(int tiles, int kblocks, double bytes, int sms, int* out) {
-  const SplitPlan plan = plan_split(tiles, kblocks, bytes, sms);
-  out[0] = plan.n_tile;
-  out[1] = plan.splits;
-}
+// Test hook (host only): the tile width that plan_narrow chooses (0: the persistent kernel).
+extern "C" int bshmem_fused_test_narrow_plan(int tiles, int kblocks, double bytes, int sms) { return plan_narrow(tiles, kblocks, bytes, sms).n_tile; }
 
 // Test hook (host only): the tile that position `t` of the tile order names, for the checks of the order's
 // invariants (every tile once, own rows last, pairs share their columns).  out = {m_tile, n_tile, peer, m_local, idx_in_peer}.

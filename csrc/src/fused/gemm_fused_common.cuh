@@ -50,7 +50,7 @@ struct alignas(64) FusedParams {
   int act;                                   // BSHMEM_FUSED_ACT_*: applied to the fp32 result in the epilogue (PLAIN / AG)
   int red_rows;                              // switch path: rows per work item of the reducing warps (16 or 32)
   int row_blocks;                            // one PE: 128-row blocks that the tile order counts (pairs: rounded up to an even number; 0: as many as there are rows)
-  int tile_end;                              // one PE: tiles of the order that this kernel computes (0: all); gemm_split_kernel follows for the rest
+  int tile_end;                              // one PE: tiles of the order that this kernel computes (0: all); gemm_narrow_kernel follows for the rest
   int a_mn, b_mn;                            // operand is stored with K outermost ([K][M] / [K][N]): loaded as it lies, no transpose pass
   int sw_reduce;                             // RS/AR: partial tiles stay local and the owner fetches their sum through the switch
 };

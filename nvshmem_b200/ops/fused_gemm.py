@@ -114,7 +114,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, max_
          w_t: bool = False) -> torch.Tensor:
     """``act(x[M,K] @ w[N,K].T)`` -> bf16 ``[M,N]`` on the tcgen05/TMEM kernel; ``act`` is None or ``"gelu_tanh"``
     (applied to the fp32 accumulators in the epilogue).  ``x_t`` / ``w_t``: the operand is stored transposed, ``x[K,M]`` /
-    ``w[K,N]`` (contiguous); the kernel reads it as it lies."""
+    ``w[K,N]`` (contiguous); the kernel reads it as it lies.  Every element is summed over K in one order in fp32, whatever
+    ``M``, ``N`` and ``max_ctas`` are: a part of the rows or of the weights gives the bits of the whole product."""
     _check_operands(x, w, x_t, w_t)
     K, M = x.shape if x_t else x.shape[::-1]
     N = w.shape[1 if w_t else 0]

@@ -121,8 +121,7 @@ def test_gemm_reads_transposed_operands_as_they_lie(M, N, K, x_t, w_t):
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (128, 256, 128), (128, 1024, 2048), (256, 512, 8192), (128, 3584, 8128), (384, 1536, 704), (512, 3584, 1984), (1152, 2816, 192),
                                    (128, 8192, 3584), (1280, 2816, 1984)])
 def test_products_of_few_tiles(M, N, K, act):
-    """Narrow tiles with K divided over a cluster (1 to 8 parts, even and uneven), the single wave it has to fit and the persistent
-    kernel beyond.  fp32 sums in another order differ by about sqrt(K) 2^-24 of the operands' scale, far below the
+    """Tiles of 64, 128 and 256 columns, the single wave they have to fit and the persistent kernel beyond.  fp32 sums in another order differ by about sqrt(K) 2^-24 of the operands' scale, far below the
     rounding to bf16 (2^-8 of the value at most)."""
     from nvshmem_b200.ops import fused_gemm as fg
     torch.manual_seed(M + N + K)
@@ -140,6 +139,26 @@ def test_products_of_few_tiles(M, N, K, act):
         fg.check_errors()
         assert bool(((got.double() - want).abs() <= want.abs() * 2 ** -8 + room).all()), (x_t, w_t)
     assert torch.equal(fg.gemm(x, w, act=act), fg.gemm(x, w, act=act))
+
+
+@pytest.mark.parametrize("M,N,K,act", [(128, 1024, 2048, None), (256, 512, 8192, "gelu_tanh"), (512, 3584, 1024, None), (1024, 1024, 1024, None), (2048, 2560, 4096, None),
+                                       (4096, 3584, 2048, "gelu_tanh")])
+def test_bits_of_a_row_do_not_depend_on_the_size_of_the_call(M, N, K, act):
+    """One chain of sums over K for every element: a part of the rows or of the weights gives the bits that the whole product
+    has, whichever kernel and tile width each of them takes (few tiles, one CTA, pairs, a last wave cut finer)."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(M + N + K)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    whole = fg.gemm(x, w, act=act)
+    assert torch.equal(whole[:128], fg.gemm(x[:128], w, act=act, max_ctas=1))
+    for rows in {128, M // 2 // 128 * 128} - {0}:
+        assert torch.equal(whole[:rows], fg.gemm(x[:rows], w, act=act)), rows
+        assert torch.equal(whole[M - rows:], fg.gemm(x[M - rows:], w, act=act)), rows
+    for cols in (256, N // 2 // 256 * 256):
+        assert torch.equal(whole[:, N - cols:], fg.gemm(x, w[N - cols:], act=act)), cols
+    assert torch.equal(whole, fg.gemm(x.t().contiguous(), w.t().contiguous(), act=act, x_t=True, w_t=True))
+    fg.check_errors()
 
 
 @pytest.mark.parametrize("M,N,K,act", [(2176, 2304, 192, None), (4480, 3584, 128, "gelu_tanh"), (2048, 4864, 1024, None), (3328, 3072, 2048, None), (1152, 8448, 64, None)])

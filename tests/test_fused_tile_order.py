@@ -110,22 +110,13 @@ def test_switch_path_walks_the_output_in_one_order_on_every_pe(mode, npes, M, N)
             assert a[1] == b[1] and a[2] == b[2] and b[0] == a[0] + 1
 
 
-def test_split_plan_fits_one_wave_and_gives_every_part_some_k():
-    """The plan of the kernel for few tiles: one wave of CTAs, at least one K step per part, widths that divide 256; no plan
-    when the tiles alone do not fit."""
+def test_narrow_plan_fits_one_wave():
+    """The plan of the kernel for few tiles: one wave of CTAs, the narrowest width that fits it; no plan when the tiles alone do
+    not fit."""
     lib = _lib()
-    lib.bshmem_fused_test_split_plan.argtypes = [C.c_int, C.c_int, C.c_double, C.c_int, C.POINTER(C.c_int)]
-    out = (C.c_int * 2)()
-    seen = set()
+    lib.bshmem_fused_test_narrow_plan.argtypes = [C.c_int, C.c_int, C.c_double, C.c_int]
     for sms in (132, 148):
         for tiles in list(range(1, 152)) + [296, 1000]:
             for kblocks in (1, 2, 3, 7, 8, 31, 128, 1000):
-                lib.bshmem_fused_test_split_plan(tiles, kblocks, 2e6, sms, out)
-                width, parts = out
-                if tiles > sms:
-                    assert width == 0
-                    continue
-                assert width in (64, 128, 256) and parts in (1, 2, 4, 8) and parts <= kblocks
-                assert tiles * (256 // width) * parts <= (sms * 7 // 16 if parts == 8 else sms * 7 // 8 if parts == 4 else sms)
-                seen.add((width, parts))
-    assert {(64, 1), (64, 4), (128, 1), (256, 1)} <= seen
+                width = lib.bshmem_fused_test_narrow_plan(tiles, kblocks, 2e6, sms)
+                assert width == next((w for w in (64, 128, 256) if tiles * (256 // w) <= sms), 0), (tiles, kblocks, sms)
