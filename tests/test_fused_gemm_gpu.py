@@ -183,6 +183,22 @@ def test_odd_row_blocks_in_pairs_and_a_last_wave_cut_finer(M, N, K, act):
         assert bool((guard[M:] == 7.0).all()), "rows past the output were written"
 
 
+@pytest.mark.parametrize("M,N,K", [(4224, 8192, 64), (4224, 8192, 128), (8320, 8192, 64), (8320, 8192, 128), (4480, 3584, 64)])
+def test_added_row_blocks_leave_the_staging_buffers_alone(M, N, K):
+    """Short K: the next accumulator is ready at once, so the tile after a stored one finds its last store still in flight.  Every
+    element against float64, new inputs every time."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+    for _ in range(60):
+        x = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+        w = (torch.randn(N, K, device="cuda", generator=gen) * 0.05).to(torch.bfloat16)
+        got = fg.gemm(x, w)
+        want = x.double() @ w.double().t()
+        # one rounding to bf16 (2^-8 of the value), K products of 2^-24 each of the largest sum
+        assert bool(((got.double() - want).abs() <= want.abs() * 2 ** -8 + K * 2.0 ** -24 * want.abs().max()).all())
+    fg.check_errors()
+
+
 def test_gemm_is_a_threads_first_cuda_call():
     """A thread that has not touched the GPU before (as an autograd worker may not have) calls the GEMM first."""
     import threading

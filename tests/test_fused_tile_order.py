@@ -120,3 +120,34 @@ def test_narrow_plan_fits_one_wave():
             for kblocks in (1, 2, 3, 7, 8, 31, 128, 1000):
                 width = lib.bshmem_fused_test_narrow_plan(tiles, kblocks, 2e6, sms)
                 assert width == next((w for w in (64, 128, 256) if tiles * (256 // w) <= sms), 0), (tiles, kblocks, sms)
+
+
+def _overwritten(staged_and_stored):
+    """Replays the epilogue's staging of one CTA: per tile (chunks staged, chunks stored).  Before a chunk writes buffer `counter & 1`, all
+    groups but the newest have been read.  Returns how often a buffer is written that a store may still be reading."""
+    bad, counter, pending = 0, 0, []          # pending: the buffer of every committed group, oldest first
+    for staged, stored in staged_and_stored:
+        for c in range(staged):
+            pending = pending[-1:]
+            bad += (counter & 1) in pending
+            if c < stored:
+                pending.append(counter & 1)
+            counter += 1
+    return bad
+
+
+@pytest.mark.parametrize("M,N", [(4224, 8192), (8320, 8192), (4480, 3584), (1152, 8448), (2176, 2304), (8192, 8192)])
+def test_no_staging_buffer_is_written_while_a_store_reads_it(M, N):
+    """Row blocks rounded up to pairs, tiles dealt to 148 CTAs as the persistent kernel deals them: the added block stages nothing.
+    Were its chunks staged and not stored, buffers would be overwritten."""
+    lib = _lib()
+    lib.bshmem_fused_test_staged_chunks.argtypes = [C.c_int] * 4
+    blocks = M // BM + (M // BM) % 2
+    total, odd = blocks * (N // BN), (M // BM) % 2
+    chunks = [lib.bshmem_fused_test_staged_chunks(M, N, blocks, t) for t in range(total)]
+    assert lib.bshmem_fused_test_staged_chunks(M, N, blocks, total) == -1
+    assert chunks.count(4) == M // BM * (N // BN) and chunks.count(0) == odd * (N // BN) and len(chunks) == total
+    per_cta = [chunks[first::148] for first in range(148)]
+    assert sum(_overwritten([(c, c) for c in tiles]) for tiles in per_cta) == 0
+    planted = sum(_overwritten([(4, c) for c in tiles]) for tiles in per_cta)
+    assert (planted > 0) == any(a == 4 and b == 0 for tiles in per_cta for a, b in zip(tiles, tiles[1:]))
