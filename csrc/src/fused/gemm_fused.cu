@@ -543,6 +543,9 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   if (a->M <= 0 || a->N <= 0 || a->K <= 0 || (!grouped && a->M % (BM * npes)) || a->N % BN || a->K % BK) return BSHMEM_FUSED_ERR_SHAPE;
   FusedParams p;
   memset(&p, 0, sizeof(p));
+  p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
+  p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
+  if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (p.a_mn && npes > 1) || (layout && grouped)) return BSHMEM_FUSED_ERR_ARGS;
   p.M = a->M; p.N = a->N; p.K = a->K; p.rank = a->rank; p.npes = npes; p.mode = mode;
   p.epoch = a->epoch;
   if (a->act != BSHMEM_FUSED_ACT_NONE && a->act != BSHMEM_FUSED_ACT_GELU_TANH && !(a->act == BSHMEM_FUSED_ACT_SWIGLU && mode == BSHMEM_FUSED_GROUPED)) return BSHMEM_FUSED_ERR_ARGS;
@@ -557,9 +560,6 @@ static int launch_gemm(const bshmem_fused_args_t* a, int layout, cudaStream_t st
   int grid = a->max_ctas > 0 && a->max_ctas < sms ? a->max_ctas : sms;
   // A pair takes two consecutive 128-row tiles of one PE's block of rows.
   bool pair = pair_wanted() && rows_per_pe % (2 * BM) == 0 && grid >= 2;
-  p.a_mn = (layout & BSHMEM_FUSED_A_TRANSPOSED) != 0;
-  p.b_mn = (layout & BSHMEM_FUSED_B_TRANSPOSED) != 0;
-  if ((layout & ~(BSHMEM_FUSED_A_TRANSPOSED | BSHMEM_FUSED_B_TRANSPOSED)) || (p.a_mn && npes > 1)) return BSHMEM_FUSED_ERR_ARGS;
   if (grouped) return launch_grouped(a, grid, p.wait_limit_ns, stream);
   // Time of the persistent kernel per K step and wave (us): 0.36 for single CTAs, 0.29 for pairs.
   const int tmr = rows_per_pe / BM, tiles_n = a->N / BN, kblocks = a->K / BK;

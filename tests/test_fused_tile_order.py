@@ -151,3 +151,15 @@ def test_no_staging_buffer_is_written_while_a_store_reads_it(M, N):
     assert sum(_overwritten([(c, c) for c in tiles]) for tiles in per_cta) == 0
     planted = sum(_overwritten([(4, c) for c in tiles]) for tiles in per_cta)
     assert (planted > 0) == any(a == 4 and b == 0 for tiles in per_cta for a, b in zip(tiles, tiles[1:]))
+
+
+@pytest.mark.parametrize("mode,npes,layout", [("grouped", 1, 1), ("grouped", 1, 2), ("grouped", 1, 3), ("plain", 1, 4), ("plain", 1, 7), ("rs", 2, 1), ("ag", 2, 3)])
+def test_layouts_that_do_not_exist_are_refused(mode, npes, layout):
+    """Transposed operands of a grouped product, unknown layout bits, A transposed with several PEs: refused by the argument
+    checks, before anything touches a GPU."""
+    _lib()  # built if it is missing
+    from nvshmem_b200.ops import fused_gemm as fg
+    a = fg._Args()
+    a.A = a.B = a.out = a.error_flag = a.group_offsets = 4096
+    a.M, a.N, a.K, a.npes, a.mode, a.groups = 256, 256, 64, npes, fg.MODES[mode], 1
+    assert fg.fused_lib().bshmem_fused_gemm_layout(C.byref(a), layout, None) == 1
