@@ -90,16 +90,14 @@ class MoeDispatchCombine:
         ptr = (lambda t, q: core.peer_ptr(t, q)) if sym else (lambda t, q: t.data_ptr())
         self._peers = {q: {"recv": ptr(self.recv_raw, q), "scale": ptr(self.recv_scale, q) if self.fp8 else 0, "y": ptr(self.expert_out, q),
                            "counts": ptr(self.counts, q), "flags": ptr(self.flags, q), "dup": ptr(self.dup_src, q) if self.dedup else 0} for q in range(self.npes)}
-        # What every call passes alike (sizes, the peers' addresses of this object's buffers); a call fills in its own copy.
+        # What every call passes alike (the peers' addresses of this object's buffers, the sizes); a call fills in its own copy.
         d, c = _DispatchArgs(), _CombineArgs()
         for q in range(self.npes):
             d.recv_x[q], d.recv_scale[q], d.dup_src[q] = self._peers[q]["recv"], self._peers[q]["scale"], self._peers[q]["dup"]
             d.counts[q], d.flags[q] = self._peers[q]["counts"], self._peers[q]["flags"]
             c.y[q], c.flags[q] = self._peers[q]["y"], self._peers[q]["flags"]
-        for a in (d, c):
-            a.T, a.H, a.K, a.E, a.rank, a.npes = T, H, K, E, self.rank, self.npes
-        d.payload, d.cap_rows = int(self.fp8), self.cap_rows
-        self._dispatch_args, self._combine_args = d, c
+        d.rank, d.npes, c.rank, c.npes = self.rank, self.npes, self.rank, self.npes
+        self._dispatch_args, self._combine_args, self._sizes = d, c, None
         if sym:
             core.barrier_all()
             torch.cuda.synchronize()
@@ -114,12 +112,22 @@ class MoeDispatchCombine:
         q = self.recv_raw[:rows].view(torch.float8_e4m3fn).float().view(rows, self.H // 128, 128)
         return (q * self.recv_scale[:rows].unsqueeze(-1)).view(rows, self.H)
 
+    def _current_sizes(self) -> None:
+        """The sizes count as they stand at the call: a program may lower ``cap_rows`` (or ``T``, with shorter inputs) in between."""
+        sizes = (self.T, self.H, self.K, self.E, self.cap_rows, self.fp8)
+        if sizes != self._sizes:
+            d, c = self._dispatch_args, self._combine_args
+            d.T, d.H, d.K, d.E, d.cap_rows, d.payload = sizes
+            c.T, c.H, c.K, c.E = sizes[:4]
+            self._sizes = sizes
+
     def dispatch(self, x: torch.Tensor, topk_idx: torch.Tensor):
         if x.shape != (self.T, self.H) or x.dtype != torch.bfloat16 or not x.is_contiguous():
             raise MoeError("x must be contiguous bf16 [T, H]")
         if topk_idx.shape != (self.T, self.K) or topk_idx.dtype != torch.int32 or not topk_idx.is_contiguous():
             raise MoeError("topk_idx must be contiguous int32 [T, K]")
         self.epoch += 1
+        self._current_sizes()
         a = _DispatchArgs.from_buffer_copy(self._dispatch_args)
         a.epoch, a.wait_limit_ms = self.epoch, self.wait_limit_ms
         a.error_flag = _error_flag(self.device).data_ptr()
@@ -134,6 +142,7 @@ class MoeDispatchCombine:
     def combine(self, topk_idx: torch.Tensor, topk_weight: torch.Tensor) -> torch.Tensor:
         if topk_weight.shape != (self.T, self.K) or topk_weight.dtype != torch.float32 or not topk_weight.is_contiguous():
             raise MoeError("topk_weight must be contiguous fp32 [T, K]")
+        self._current_sizes()
         a = _CombineArgs.from_buffer_copy(self._combine_args)
         a.epoch, a.wait_limit_ms = self.epoch, self.wait_limit_ms
         a.error_flag = _error_flag(self.device).data_ptr()

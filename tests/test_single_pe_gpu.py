@@ -230,6 +230,34 @@ def test_local_combine_over_column_ranges(nv, T, H, K):
     moe.close()
 
 
+@pytest.mark.parametrize("T", [100, 700])
+def test_sizes_of_the_exchange_count_as_they_stand_at_the_call(nv, T):
+    """`cap_rows` lowered after the first call: rows beyond it are dropped and reported; `T` lowered: a shorter batch."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    from nvshmem_b200.ops.moe import MoeDispatchCombine
+    torch.manual_seed(T)
+    H, K, E = 256, 4, 8
+    moe = MoeDispatchCombine(T, H, K, E)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    idx = torch.rand(T, E, device="cuda").topk(K, dim=-1).indices.to(torch.int32).contiguous()
+    wt = torch.full((T, K), 0.25, device="cuda")
+    moe.dispatch(x, idx)
+    assert fg.take_error() == 0 and int(moe.slot_map.max()) == T * K - 1
+    moe.cap_rows = cap = T * K // 3
+    moe.recv_raw.fill_(9)
+    moe.dispatch(x, idx)
+    assert fg.take_error() == 2 and int(moe.slot_map.max()) == cap - 1 and bool((moe.recv_raw[cap:] == 9).all())
+    moe.cap_rows, moe.T = T * K, T // 2
+    recv, offsets = moe.dispatch(x[:T // 2], idx[:T // 2])
+    assert fg.take_error() == 0 and int(offsets[-1]) == T // 2 * K
+    moe.expert_out.copy_(recv)
+    moe.out.fill_(9)
+    out = moe.combine(idx[:T // 2], wt[:T // 2])
+    torch.cuda.synchronize()
+    assert torch.equal(out[:T // 2], x[:T // 2]) and bool((out[T // 2:] == 9).all())
+    moe.close()
+
+
 @pytest.mark.parametrize("T,payload", [(40, "bf16"), (1200, "bf16"), (1200, "fp8")])
 def test_captured_calls_replay_on_new_inputs(nv, T, payload):
     """Dispatch (one and two kernels), grouped GEMM, combine, a small GEMM, one with a finer last wave and a collective in one
