@@ -619,20 +619,21 @@ __global__ void __launch_bounds__(THREADS) dispatch_small_kernel(const __grid_co
   }
 }
 
-// Routing of a large batch: CTA c of the cluster takes a contiguous eighth of the pairs.  A pair's place among its CTA's pairs
-// of the same expert comes from a shared-memory counter and waits in slot_map until the starts are known.
-__global__ void __cluster_dims__(ROUTE_CTAS, 1, 1) __launch_bounds__(ROUTE_THREADS) route_kernel(const __grid_constant__ DispatchParams P) {
+// Routing of a large batch: the CTAs of one cluster (ROUTE_CTAS, or fewer where the caller allows fewer) take contiguous parts of the
+// pairs.  A pair's place among its CTA's pairs of the same expert comes from a shared-memory counter and waits in slot_map until the
+// starts are known.
+__global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const __grid_constant__ DispatchParams P) {
   namespace cg = cooperative_groups;
   const bshmem_moe_dispatch_args_t& a = P.a;
   cg::cluster_group cluster = cg::this_cluster();
   // The kernel that moves the rows may start now: it loads token rows (which nothing here writes) and waits for this grid
   // to end before it reads the slot map.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int me = (int)cluster.block_rank(), E = a.E;
+  const int me = (int)cluster.block_rank(), ctas = (int)cluster.num_blocks(), E = a.E;
   __shared__ int s_count[BSHMEM_MOE_MAX_EXPERTS], s_start[BSHMEM_MOE_MAX_EXPERTS];
   for (int e = threadIdx.x; e < E; e += ROUTE_THREADS) s_count[e] = 0;
   __syncthreads();
-  const long pairs = (long)a.T * a.K, per = (pairs + ROUTE_CTAS - 1) / ROUTE_CTAS;
+  const long pairs = (long)a.T * a.K, per = (pairs + ctas - 1) >> (__ffs(ctas) - 1);  // a power of two
   const long lo = min(pairs, per * me), hi = min(pairs, per * (me + 1));
   // The first ROUTE_HELD pairs of a thread stay in registers (all of a batch of 8192 tokens x 8), the rest goes by way of slot_map.
   constexpr int ROUTE_HELD = 8;
@@ -655,7 +656,7 @@ __global__ void __cluster_dims__(ROUTE_CTAS, 1, 1) __launch_bounds__(ROUTE_THREA
   if ((int)threadIdx.x < E) {
 #pragma unroll
     for (int c = 0; c < ROUTE_CTAS; ++c) {
-      const int v = *cluster.map_shared_rank(&s_count[threadIdx.x], c);
+      const int v = c < ctas ? *cluster.map_shared_rank(&s_count[threadIdx.x], c) : 0;
       if (c < me) before += v;
       mine += v;
     }
@@ -838,8 +839,20 @@ static int dispatch_local(DispatchParams& P, cudaStream_t stream) {
     kernel<<<grid, THREADS, 0, stream>>>(P);
     return launched("bshmem_moe_dispatch", cudaGetLastError());
   }
-  route_kernel<<<ROUTE_CTAS, ROUTE_THREADS, 0, stream>>>(P);
-  st = launched("bshmem_moe_dispatch", cudaGetLastError());
+  // `max_ctas` holds for the call: a smaller cluster routes, and the rows wait for it instead of running beside it.
+  int ctas = ROUTE_CTAS;
+  while (a.max_ctas > 0 && ctas > a.max_ctas) ctas /= 2;
+  cudaLaunchConfig_t route = {};
+  route.gridDim = dim3(ctas);
+  route.blockDim = dim3(ROUTE_THREADS);
+  route.stream = stream;
+  cudaLaunchAttribute cluster[1];
+  cluster[0].id = cudaLaunchAttributeClusterDimension;
+  cluster[0].val.clusterDim.x = ctas;
+  cluster[0].val.clusterDim.y = cluster[0].val.clusterDim.z = 1;
+  route.attrs = cluster;
+  route.numAttrs = 1;
+  st = launched("bshmem_moe_dispatch", cudaLaunchKernelEx(&route, route_kernel, P));
   if (st) return st;
   const long pieces = (a.H * 2l + PUSH_BYTES - 1) / PUSH_BYTES;
   const int threads = fp8 ? THREADS : PUSH_WARPS * 32;
@@ -857,7 +870,7 @@ static int dispatch_local(DispatchParams& P, cudaStream_t stream) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = a.max_ctas > 0 ? 0 : 1;
   return launched("bshmem_moe_dispatch", cudaLaunchKernelEx(&cfg, kernel, P));
 }
 

@@ -230,6 +230,54 @@ def test_local_combine_over_column_ranges(nv, T, H, K):
     moe.close()
 
 
+@pytest.mark.parametrize("limit", [1, 3, 4, 7, 8, 100])
+@pytest.mark.parametrize("T,payload", [(64, "bf16"), (900, "bf16"), (900, "fp8")])
+def test_max_ctas_holds_for_every_kernel_of_the_exchange(nv, T, payload, limit):
+    """The grids of a captured dispatch and combine keep to `max_ctas` (the routing kernel too), and the rows land as they do
+    without a limit."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    from nvshmem_b200.ops.moe import MoeDispatchCombine
+    torch.manual_seed(T + limit)
+    H, K, E = 256, 5, 24
+    moe = MoeDispatchCombine(T, H, K, E, payload=payload)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    idx = torch.randint(-1, E, (T, K), device="cuda", dtype=torch.int32)
+    wt = torch.rand(T, K, device="cuda")
+    valid = idx >= 0
+    moe.dispatch(x, idx)
+    want_rows = moe.recv_raw[moe.slot_map[valid].long()].clone()
+    want_offsets, want_out = moe.expert_offsets.clone(), None
+    moe.expert_out.copy_(torch.randn(moe.cap_rows, H, device="cuda"))
+    by_slot = moe.expert_out[moe.slot_map.clamp(min=0).long()].clone()
+    want_out = moe.combine(idx, wt).clone()
+    moe._dispatch_args.max_ctas = moe._combine_args.max_ctas = limit
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        moe.dispatch(x, idx)
+        moe.combine(idx, wt)
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    err, _, count = driver.cuGraphGetNodes(raw, 0)
+    err, nodes, count = driver.cuGraphGetNodes(raw, count)
+    grids = []
+    for node in nodes[:count]:
+        if driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            err, params = driver.cuGraphKernelNodeGetParams(node)
+            assert int(err) == 0
+            grids.append(params.gridDimX * params.gridDimY * params.gridDimZ)
+    assert len(grids) == (2 if T * K <= 2048 else 3) and max(grids) <= limit, grids
+    moe.dispatch(x, idx)
+    torch.cuda.synchronize()
+    assert torch.equal(moe.expert_offsets, want_offsets) and bool((moe.slot_map[~valid] == -1).all())
+    rows = moe.slot_map[valid].long()
+    e = idx[valid].long()
+    assert torch.equal(rows.sort().values, torch.arange(rows.numel(), device="cuda"))
+    assert bool(((rows >= want_offsets[e]) & (rows < want_offsets[e + 1])).all())
+    assert torch.equal(moe.recv_raw[rows], want_rows)
+    moe.expert_out[rows] = by_slot[valid]
+    assert torch.equal(moe.combine(idx, wt), want_out)
+    moe.close()
+
+
 @pytest.mark.parametrize("T", [100, 700])
 def test_sizes_of_the_exchange_count_as_they_stand_at_the_call(nv, T):
     """`cap_rows` lowered after the first call: rows beyond it are dropped and reported; `T` lowered: a shorter batch."""
