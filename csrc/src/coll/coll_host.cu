@@ -146,7 +146,8 @@ static int ctas_for(size_t bytes, size_t threshold) {
 }
 
 // ------------------------------------------------------------------ teams of one member
-// Every data collective of a team of one is a copy of its source.  Nothing has to be met or flagged, so the launch is not
+// Every data collective of a team of one is a copy of its source, unless the caller names an algorithm (that runs the kernel for
+// several members as ever, on its few CTAs).  Nothing has to be met or flagged, so the launch is not
 // tied to the rows of barrier flags (32 CTAs at most) and fills the GPU: bound by HBM.  256 threads keep four 16-byte
 // loads each in flight, eight CTAs fit an SM, so 128 KB per SM are on their way; a CTA takes 16 KB per round.
 // 256 MB read and 256 MB written: 213 us with 32 CTAs of 512 threads, 89 us here (6.06 TB/s).
@@ -232,7 +233,7 @@ int coll_reduce_on_stream(int team, void* dst, const void* src, size_t n, int dt
   if (!f) return ST_INVALID_VALUE;
   if (n == 0) return ST_SUCCESS;
   const size_t bytes = n * dtype_size(dtype);
-  if (team_get(team)->size == 1) {
+  if (team_get(team)->size == 1 && algo == RED_AUTO) {
     local_copy(dst, src, bytes, stream);
     return launch_status("reduce");
   }
@@ -251,7 +252,7 @@ int coll_reducescatter_on_stream(int team, void* dst, const void* src, size_t nr
   if (!f) return ST_INVALID_VALUE;
   if (nreduce == 0) return ST_SUCCESS;
   const size_t bytes = nreduce * dtype_size(dtype) * team_get(team)->size;
-  if (team_get(team)->size == 1) {
+  if (team_get(team)->size == 1 && algo == RS_AUTO) {
     local_copy(dst, src, bytes, stream);
     return launch_status("reducescatter");
   }
@@ -314,7 +315,7 @@ int coll_fcollect_on_stream(int team, void* dst, const void* src, size_t block_b
     rt().n_coll++;
     return ce_fcollect(team_get(team), dst, src, block_bytes, stream);
   }
-  if (team_get(team)->size == 1) {
+  if (team_get(team)->size == 1 && algo == FC_AUTO) {
     local_copy(dst, src, total, stream);
     return launch_status("fcollect");
   }
@@ -324,7 +325,7 @@ int coll_fcollect_on_stream(int team, void* dst, const void* src, size_t block_b
   return launch_status("fcollect");
 }
 
-int coll_alltoall_on_stream(int team, void* dst, const void* src, size_t block_bytes, cudaStream_t stream) {
+int coll_alltoall_on_stream(int team, void* dst, const void* src, size_t block_bytes, cudaStream_t stream, bool members_kernel) {
   if (host_mode()) return block_bytes ? emul_alltoall(team, dst, src, block_bytes) : ST_SUCCESS;
   NvtxRange nvtx(NVTX_COLL, "alltoall_on_stream");
   int st = check_team(team, "alltoall");
@@ -335,7 +336,7 @@ int coll_alltoall_on_stream(int team, void* dst, const void* src, size_t block_b
     rt().n_coll++;
     return ce_alltoall(team_get(team), dst, src, block_bytes, stream);
   }
-  if (team_get(team)->size == 1) {
+  if (team_get(team)->size == 1 && !members_kernel) {
     local_copy(dst, src, total, stream);
     return launch_status("alltoall");
   }
@@ -355,7 +356,7 @@ int coll_broadcast_on_stream(int team, void* dst, const void* src, size_t bytes,
     rt().n_coll++;
     return ce_broadcast(team_get(team), dst, src, bytes, root, stream);
   }
-  if (team_get(team)->size == 1) {
+  if (team_get(team)->size == 1 && algo == BC_AUTO) {
     local_copy(dst, src, bytes, stream);
     return launch_status("broadcast");
   }

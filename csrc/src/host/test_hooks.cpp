@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../bootstrap/bootstrap.h"
+#include "../coll/coll_host.h"
 #include "../heap/allocator.h"
 #include "../util/env.h"
 #include "../util/log.h"
@@ -16,6 +17,10 @@ using namespace bshmem;
 
 extern "C" {
 
+// The all-to-all kernel for several members on a team of one, which otherwise copies (the other collectives take an algorithm).
+int bshmem_test_alltoall_kernel(int team, void* dst, const void* src, size_t block_bytes, cudaStream_t stream) {
+  return coll_alltoall_on_stream(team, dst, src, block_bytes, stream, true);
+}
 int bshmem_test_parse_size(const char* text, unsigned long long* out) {
   size_t v = 0;
   bool ok = parse_size(text, &v);

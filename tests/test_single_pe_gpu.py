@@ -84,6 +84,55 @@ def test_collectives_of_one_member_copy_every_byte_and_no_more(nv, n, so, do):
     nv.free_tensor(dst)
 
 
+def _kernels(call):
+    """(name, CTAs) of every kernel that `call` launches on the current stream, in order."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = driver.cuGraphGetNodes(raw, driver.cuGraphGetNodes(raw, 0)[2])[1]
+    out = []
+    for node in nodes:
+        if driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            err, p = driver.cuGraphKernelNodeGetParams(node)
+            assert int(err) == 0
+            err, name = driver.cuFuncGetName(p.func) if int(p.func) else driver.cuKernelGetName(p.kern)
+            assert int(err) == 0
+            out.append((name.decode(), p.gridDimX * p.gridDimY * p.gridDimZ))
+    return out
+
+
+@pytest.mark.parametrize("dtype,n", [(torch.float32, 1), (torch.bfloat16, 4099), (torch.int32, 70001), (torch.float64, 1 << 20)])
+def test_a_named_algorithm_runs_its_kernel_on_a_team_of_one(nv, dtype, n):
+    """The kernels for several members, which the automatic choice leaves aside for one member: reachable by naming an algorithm
+    (the all-to-all through a test hook), same bytes as the copy kernel, nothing written beyond."""
+    import ctypes as C
+    from nvshmem_b200.bindings import host as H
+    src, dst = nv.tensor((n + 8,), dtype), nv.tensor((n + 8,), dtype)
+    src.copy_((torch.arange(n + 8, device="cuda") % 113).to(dtype))
+
+    def alltoall_kernel():
+        assert H.load().bshmem_test_alltoall_kernel(0, C.c_void_p(dst.data_ptr()), C.c_void_p(src.data_ptr()), C.c_size_t(n * src.element_size()),
+                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+
+    calls = [("reduce_kernel", lambda a=a: nv.reduce(0, dst[:n], src[:n], "sum", algo=a)) for a in ("oneshot", "twoshot", "ll", "ll128", "recexch")]
+    calls += [("reducescatter_kernel", lambda: nv.reducescatter(0, dst[:n], src[:n], "sum", algo="pull"))]
+    calls += [("fcollect_kernel", lambda a=a: nv.fcollect(0, dst[:n], src[:n], algo=a)) for a in ("push", "ll", "ll128")]
+    calls += [("broadcast_kernel", lambda a=a: nv.broadcast(0, dst[:n], src[:n], algo=a)) for a in ("push", "pull", "ll")]
+    calls += [("alltoall_kernel", alltoall_kernel), ("local_copy_kernel", lambda: nv.reduce(0, dst[:n], src[:n], "sum"))]
+    for kernel, call in calls:
+        dst.fill_(7)
+        call()
+        torch.cuda.synchronize()
+        assert torch.equal(dst[:n], src[:n]) and bool((dst[n:] == 7).all()), kernel
+        names = _kernels(call)
+        assert len(names) == 1 and kernel in names[0][0], (kernel, names)
+    assert nv.error_bits() == 0
+    nv.free_tensor(src)
+    nv.free_tensor(dst)
+
+
 def test_signal_and_wait_on_stream(nv):
     sig = nv.tensor((1,), torch.int64, zero=True)
     nv.signal_op(sig, 5, nv.SignalOp.SIGNAL_SET, 0)
@@ -235,7 +284,6 @@ def test_local_combine_over_column_ranges(nv, T, H, K):
 def test_max_ctas_holds_for_every_kernel_of_the_exchange(nv, T, payload, limit):
     """The grids of a captured dispatch and combine keep to `max_ctas` (the routing kernel too), and the rows land as they do
     without a limit."""
-    driver = pytest.importorskip("cuda.bindings.driver")
     from nvshmem_b200.ops.moe import MoeDispatchCombine
     torch.manual_seed(T + limit)
     H, K, E = 256, 5, 24
@@ -251,19 +299,7 @@ def test_max_ctas_holds_for_every_kernel_of_the_exchange(nv, T, payload, limit):
     by_slot = moe.expert_out[moe.slot_map.clamp(min=0).long()].clone()
     want_out = moe.combine(idx, wt).clone()
     moe._dispatch_args.max_ctas = moe._combine_args.max_ctas = limit
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph):
-        moe.dispatch(x, idx)
-        moe.combine(idx, wt)
-    raw = driver.CUgraph(graph.raw_cuda_graph())
-    err, _, count = driver.cuGraphGetNodes(raw, 0)
-    err, nodes, count = driver.cuGraphGetNodes(raw, count)
-    grids = []
-    for node in nodes[:count]:
-        if driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
-            err, params = driver.cuGraphKernelNodeGetParams(node)
-            assert int(err) == 0
-            grids.append(params.gridDimX * params.gridDimY * params.gridDimZ)
+    grids = [ctas for _, ctas in _kernels(lambda: (moe.dispatch(x, idx), moe.combine(idx, wt)))]
     assert len(grids) == (2 if T * K <= 2048 else 3) and max(grids) <= limit, grids
     moe.dispatch(x, idx)
     torch.cuda.synchronize()
