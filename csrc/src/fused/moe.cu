@@ -888,7 +888,8 @@ static int check_common(int T, int H, int K, int E, int rank, int npes) {
   return 0;
 }
 
-extern "C" int bshmem_moe_dispatch(const bshmem_moe_dispatch_args_t* a, cudaStream_t stream) {
+// `general`: the kernel for several PEs also with one.
+static int dispatch(const bshmem_moe_dispatch_args_t* a, bool general, cudaStream_t stream) {
   if (!a || !a->x || !a->topk_idx || !a->slot_map || !a->expert_offsets || !a->scratch || !a->error_flag) return BSHMEM_MOE_ERR_ARGS;
   int st = check_common(a->T, a->H, a->K, a->E, a->rank, a->npes);
   if (st) return st;
@@ -897,7 +898,7 @@ extern "C" int bshmem_moe_dispatch(const bshmem_moe_dispatch_args_t* a, cudaStre
   DispatchParams P;
   P.a = *a;
   P.wait_limit_ns = a->wait_limit_ms ? (uint64_t)a->wait_limit_ms * 1000000ull : 10000000000ull;
-  if (a->npes == 1 && !a->dup_src[0]) return dispatch_local(P, stream);
+  if (a->npes == 1 && !a->dup_src[0] && !general) return dispatch_local(P, stream);
   const size_t smem = dispatch_smem(a->E, a->H);
   int grid = 0;
   st = coop_grid(dispatch_kernel, smem, a->T, a->max_ctas, &grid);
@@ -912,7 +913,7 @@ extern "C" int bshmem_moe_dispatch(const bshmem_moe_dispatch_args_t* a, cudaStre
   return 0;
 }
 
-extern "C" int bshmem_moe_combine(const bshmem_moe_combine_args_t* a, cudaStream_t stream) {
+static int combine(const bshmem_moe_combine_args_t* a, bool general, cudaStream_t stream) {
   if (!a || !a->topk_idx || !a->topk_weight || !a->slot_map || !a->out || !a->scratch || !a->error_flag) return BSHMEM_MOE_ERR_ARGS;
   int st = check_common(a->T, a->H, a->K, a->E, a->rank, a->npes);
   if (st) return st;
@@ -923,7 +924,7 @@ extern "C" int bshmem_moe_combine(const bshmem_moe_combine_args_t* a, cudaStream
   P.wait_limit_ns = a->wait_limit_ms ? (uint64_t)a->wait_limit_ms * 1000000ull : 10000000000ull;
   int grid = 0;
   P.split = 1;
-  if (a->npes == 1) {
+  if (a->npes == 1 && !general) {
     P.split = column_split(a->T, a->H / BSHMEM_MOE_QUANT_BLOCK);
     const bool narrow = (a->H / 8 + P.split - 1) / P.split <= THREADS / 2;
     auto kernel = a->K <= 8 ? (narrow ? combine_kernel<8, true, true> : combine_kernel<8, true, false>)
@@ -946,6 +947,12 @@ extern "C" int bshmem_moe_combine(const bshmem_moe_combine_args_t* a, cudaStream
   }
   return 0;
 }
+
+extern "C" int bshmem_moe_dispatch(const bshmem_moe_dispatch_args_t* a, cudaStream_t stream) { return dispatch(a, false, stream); }
+extern "C" int bshmem_moe_combine(const bshmem_moe_combine_args_t* a, cudaStream_t stream) { return combine(a, false, stream); }
+// Test hooks: the kernels for several PEs on one PE, which otherwise takes kernels of its own.
+extern "C" int bshmem_moe_test_dispatch_general(const bshmem_moe_dispatch_args_t* a, cudaStream_t stream) { return dispatch(a, true, stream); }
+extern "C" int bshmem_moe_test_combine_general(const bshmem_moe_combine_args_t* a, cudaStream_t stream) { return combine(a, true, stream); }
 
 // ------------------------------------------------------------------ dispatch without any allocation
 // Single-PE dispatch whose scratch is a fixed array inside this library (see bshmem/moe_noalloc.h

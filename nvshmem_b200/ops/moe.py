@@ -39,10 +39,10 @@ class _CombineArgs(C.Structure):
 def _lib():
     lib = fused_lib()
     if not hasattr(lib, "_moe_ready"):
-        lib.bshmem_moe_dispatch.restype = C.c_int
-        lib.bshmem_moe_dispatch.argtypes = [C.POINTER(_DispatchArgs), C.c_void_p]
-        lib.bshmem_moe_combine.restype = C.c_int
-        lib.bshmem_moe_combine.argtypes = [C.POINTER(_CombineArgs), C.c_void_p]
+        for fn in (lib.bshmem_moe_dispatch, lib.bshmem_moe_test_dispatch_general):
+            fn.restype, fn.argtypes = C.c_int, [C.POINTER(_DispatchArgs), C.c_void_p]
+        for fn in (lib.bshmem_moe_combine, lib.bshmem_moe_test_combine_general):
+            fn.restype, fn.argtypes = C.c_int, [C.POINTER(_CombineArgs), C.c_void_p]
         lib.bshmem_moe_scratch_bytes.restype = C.c_size_t
         lib.bshmem_moe_scratch_bytes.argtypes = [C.c_int]
         lib._moe_ready = True
@@ -98,6 +98,7 @@ class MoeDispatchCombine:
             c.y[q], c.flags[q] = self._peers[q]["y"], self._peers[q]["flags"]
         d.rank, d.npes, c.rank, c.npes = self.rank, self.npes, self.rank, self.npes
         self._dispatch_args, self._combine_args, self._sizes = d, c, None
+        self._use_kernels_for_several_pes(False)
         if sym:
             core.barrier_all()
             torch.cuda.synchronize()
@@ -111,6 +112,12 @@ class MoeDispatchCombine:
         """fp8 payload back to fp32 (tests and reference expert MLPs)."""
         q = self.recv_raw[:rows].view(torch.float8_e4m3fn).float().view(rows, self.H // 128, 128)
         return (q * self.recv_scale[:rows].unsqueeze(-1)).view(rows, self.H)
+
+    def _use_kernels_for_several_pes(self, always: bool) -> None:
+        """One PE has kernels of its own; tests and profiles reach the others with ``always``."""
+        lib = _lib()
+        self._dispatch_entry = lib.bshmem_moe_test_dispatch_general if always else lib.bshmem_moe_dispatch
+        self._combine_entry = lib.bshmem_moe_test_combine_general if always else lib.bshmem_moe_combine
 
     def _current_sizes(self) -> None:
         """The sizes count as they stand at the call: a program may lower ``cap_rows`` (or ``T``, with shorter inputs) in between."""
@@ -134,7 +141,7 @@ class MoeDispatchCombine:
         a.x, a.topk_idx = x.data_ptr(), topk_idx.data_ptr()
         a.slot_map, a.expert_offsets, a.src_offsets = self.slot_map.data_ptr(), self.expert_offsets.data_ptr(), self.src_offsets.data_ptr()
         a.scratch = self.scratch.data_ptr()
-        st = _lib().bshmem_moe_dispatch(C.byref(a), C.c_void_p(H.current_stream_handle()))
+        st = self._dispatch_entry(C.byref(a), C.c_void_p(H.current_stream_handle()))
         if st != 0:
             raise MoeError(f"bshmem_moe_dispatch failed with status {st}")
         return self.recv_x, self.expert_offsets
@@ -148,7 +155,7 @@ class MoeDispatchCombine:
         a.error_flag = _error_flag(self.device).data_ptr()
         a.topk_idx, a.topk_weight, a.slot_map, a.out = topk_idx.data_ptr(), topk_weight.data_ptr(), self.slot_map.data_ptr(), self.out.data_ptr()
         a.scratch = self.scratch.data_ptr()
-        st = _lib().bshmem_moe_combine(C.byref(a), C.c_void_p(H.current_stream_handle()))
+        st = self._combine_entry(C.byref(a), C.c_void_p(H.current_stream_handle()))
         if st != 0:
             raise MoeError(f"bshmem_moe_combine failed with status {st}")
         return self.out

@@ -279,6 +279,56 @@ def test_local_combine_over_column_ranges(nv, T, H, K):
     moe.close()
 
 
+@pytest.mark.parametrize("payload", ["bf16", "fp8"])
+@pytest.mark.parametrize("T,H,K,E", [(1, 128, 1, 8), (61, 7168, 8, 32), (300, 256, 16, 64), (700, 2176, 9, 16), (5000, 128, 4, 256)])
+def test_exchange_of_several_pes_run_on_one(nv, T, H, K, E, payload):
+    """The kernels that several PEs run (cooperative, with barriers), on one PE against the ones without barriers: same
+    offsets, same rows per token, and the same bits from combine (builds for up to 8 and up to 16 choices)."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    from nvshmem_b200.ops.moe import MoeDispatchCombine
+    torch.manual_seed(T + H)
+    x = torch.randn(T, H, device="cuda").to(torch.bfloat16)
+    idx = torch.randint(-1, E, (T, K), device="cuda", dtype=torch.int32)
+    wt = torch.rand(T, K, device="cuda")
+    rows = torch.randn(T, K, H, device="cuda").to(torch.bfloat16)  # an expert's answer for every (token, choice)
+    valid = idx >= 0
+    res = []
+    for several in (False, True):
+        moe = MoeDispatchCombine(T, H, K, E, payload=payload)
+        moe._use_kernels_for_several_pes(several)
+        for _ in range(2):  # the second call finds what the first one left in flags and scratch
+            recv, offsets = moe.dispatch(x, idx)
+            at = moe.slot_map[valid].long()
+            moe.expert_out[at] = rows[valid]
+            out = moe.combine(idx, wt)
+        names = [n for n, _ in _kernels(lambda: (moe.dispatch(x, idx), moe.combine(idx, wt)))]
+        assert ("15dispatch_kernel" in names[0]) == several, names
+        fg.check_errors()
+        res.append((offsets.clone(), recv.view(torch.uint8)[at].clone(), moe.recv_scale[at].clone() if payload == "fp8" else None, moe.src_offsets.clone(), out.clone()))
+        moe.close()
+    one, general = res
+    for k in (0, 1, 3, 4):
+        assert torch.equal(one[k], general[k]), k
+    if payload == "fp8":
+        assert torch.equal(one[2], general[2])
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 512, 192), (1152, 2048, 64)])
+def test_fused_ops_with_a_transposed_weight(nv, M, N, K):
+    """``w_t=True`` of the ops that the backward passes on several PEs use, on one."""
+    from nvshmem_b200.ops import fused_gemm as fg
+    torch.manual_seed(M)
+    x = torch.randn(M, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    want = fg.gemm(x, w)
+    ag = fg.AllGatherGemm(M, K)
+    ag.shard.copy_(x)
+    for got in (ag(w.t().contiguous(), w_t=True), fg.GemmReduceScatter(M, N, mode="rs")(x, w.t().contiguous(), w_t=True),
+                fg.GemmReduceScatter(M, N, mode="ar")(x, w.t().contiguous(), w_t=True)):
+        assert torch.equal(got, want)
+    fg.check_errors()
+
+
 @pytest.mark.parametrize("limit", [1, 3, 4, 7, 8, 100])
 @pytest.mark.parametrize("T,payload", [(64, "bf16"), (900, "bf16"), (900, "fp8")])
 def test_max_ctas_holds_for_every_kernel_of_the_exchange(nv, T, payload, limit):
