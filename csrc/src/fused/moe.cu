@@ -399,8 +399,10 @@ __device__ __forceinline__ void combine_token(const uint8_t* const* src, const f
 // H 128, top-4, 16364 tokens: 36.6 -> 6.7 us.
 // NARROW: rows (or column ranges) of at most half as many 16-byte pieces as the CTA has threads are taken several at a time,
 // a power of two of threads each; a build of its own because the variable stride costs wide rows 3 %.
+// The bound of one CTA more per SM is for LOCAL alone, where it was measured; the others keep the registers that hold their loads in
+// flight (62 and 85, against 54 and 79; 4096 tokens of 128 values, top-8, on one PE 24.5 us against 26.6).
 template <int KT, bool LOCAL, bool NARROW>
-__global__ void __launch_bounds__(THREADS, KT <= 8 ? 4 : 3) combine_kernel(const __grid_constant__ CombineParams P) {
+__global__ void __launch_bounds__(THREADS, (KT <= 8 ? 3 : 2) + (LOCAL ? 1 : 0)) combine_kernel(const __grid_constant__ CombineParams P) {
   const bshmem_moe_combine_args_t& a = P.a;
   const int H = a.H, K = a.K, E = a.E, npes = a.npes, rank = a.rank;
   const int EL = E / npes;
@@ -934,7 +936,7 @@ static int combine(const bshmem_moe_combine_args_t* a, bool general, cudaStream_
     kernel<<<grid, THREADS, 0, stream>>>(P);
     return launched("bshmem_moe_combine", cudaGetLastError());
   }
-  // Two builds of the kernel: up to 8 choices per token (fewer registers, three CTAs per SM) and up to 16.
+  // Two builds of the kernel: up to 8 choices per token (62 registers, four CTAs per SM) and up to 16 (85, two).
   const void* kernel = a->K <= 8 ? (const void*)combine_kernel<8, false, false> : (const void*)combine_kernel<BSHMEM_MOE_MAX_TOPK, false, false>;
   st = a->K <= 8 ? coop_grid(combine_kernel<8, false, false>, 0, a->T, a->max_ctas, &grid) : coop_grid(combine_kernel<BSHMEM_MOE_MAX_TOPK, false, false>, 0, a->T, a->max_ctas, &grid);
   if (st) return st;
