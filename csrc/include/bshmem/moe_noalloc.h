@@ -7,8 +7,8 @@
 // under a memory-accounting sandbox, or a latency-critical path where an
 // allocation could stall behind another thread's free.  Such a caller can hand
 // over its own input and output buffers but has nowhere to get the small
-// scratch block (counters and a barrier word) that the MoE dispatch kernel
-// needs.  Here that block lives inside the library, in a fixed array in device
+// block (the experts' row counts and an error word) that the MoE dispatch
+// writes besides.  Here that block lives inside the library, in a fixed array in device
 // memory that exists from the moment the library is loaded on a GPU until the
 // process ends.
 //
@@ -23,12 +23,12 @@
 //   * experts <= BSHMEM_MOE_NOALLOC_MAX_EXPERTS (1024), top-k <= 16, H a multiple of 128;
 //     anything beyond is refused with BSHMEM_MOE_ERR_SHAPE and a message on stderr.
 //   * `recv_x` must hold T*K rows of H bf16 values.
-//   * The built-in scratch is about 13 KB per GPU (BSHMEM_MOE_NOALLOC_SCRATCH_BYTES).
+//   * The built-in array takes BSHMEM_MOE_NOALLOC_SCRATCH_BYTES (13 KB) per GPU, of which a little over 4 KB are in use.
 //   * The first call on a GPU looks up the array's device address; make that first call
 //     outside any CUDA stream capture, with the GPU current.
 //   * Every call on a GPU shares the one array: calls whose kernels could overlap on the
 //     GPU (different streams, no ordering between them) race.  Issue them on one stream
-//     or order them yourself.  Each call clears the words that must start at zero.
+//     or order them yourself.  Each call clears the error word, writes all counts, and needs nothing else.
 //   * Errors that the kernel meets (BSHMEM_MOE_ERRBIT_*) go to the caller's `error_flag`.  A caller that passes
 //     none does not lose them: they go to a word inside the built-in array, which
 //     bshmem_moe_noalloc_error_bits() reads back (it waits for the stream first).  The next call on the

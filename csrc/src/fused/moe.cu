@@ -957,8 +957,8 @@ extern "C" int bshmem_moe_test_dispatch_general(const bshmem_moe_dispatch_args_t
 extern "C" int bshmem_moe_test_combine_general(const bshmem_moe_combine_args_t* a, cudaStream_t stream) { return combine(a, true, stream); }
 
 // ------------------------------------------------------------------ dispatch without any allocation
-// Single-PE dispatch whose scratch is a fixed array inside this library (see bshmem/moe_noalloc.h
-// for who needs that and the rules of use).  In host code the array's name is only a handle; the
+// Single-PE dispatch whose count matrix and error word are a fixed array inside this library (see
+// bshmem/moe_noalloc.h for who needs that and the rules of use).  In host code the array's name is only a handle; the
 // address a kernel can use comes from cudaGetSymbolAddress, looked up once per GPU.
 #include <limits.h>
 
@@ -969,11 +969,8 @@ extern "C" int bshmem_moe_test_combine_general(const bshmem_moe_combine_args_t* 
 namespace {
 
 struct NoAllocBlock {
-  bshmem::moe::Scratch scratch;                    // counters + grid-barrier word (cleared every call)
-  int counts[BSHMEM_MOE_NOALLOC_MAX_EXPERTS];      // the 1 x E count matrix
-  uint64_t flags[4];                               // cross-PE barrier rows (unused with one PE, must exist)
-  int error_flag;                                  // used when the caller passes none
-  int pad[7];
+  int counts[BSHMEM_MOE_NOALLOC_MAX_EXPERTS];  // the 1 x E count matrix (the kernels write all E of them)
+  int error_flag;                              // used when the caller passes none; cleared by every call
 };
 static_assert(sizeof(NoAllocBlock) <= BSHMEM_MOE_NOALLOC_SCRATCH_BYTES, "documented scratch size is too small");
 
@@ -1018,8 +1015,8 @@ extern "C" int bshmem_moe_dispatch_local_noalloc(const void* x, const int* topk_
   NoAllocBlock* blk = nullptr;
   int bst = noalloc_block(&blk);
   if (bst) return bst;
-  // The block keeps what the previous call left: clear the counters, the barrier word, the flags and the built-in error word.
-  if (cudaMemsetAsync(blk, 0, sizeof(NoAllocBlock), stream) != cudaSuccess) return BSHMEM_MOE_ERR_DRIVER;
+  // Of what the previous call left, only the error word has to start at zero (a caller with a word of its own may still ask for it).
+  if (cudaMemsetAsync(&blk->error_flag, 0, sizeof(int), stream) != cudaSuccess) return BSHMEM_MOE_ERR_DRIVER;
 
   DispatchParams P;
   memset(&P, 0, sizeof(P));
@@ -1036,8 +1033,6 @@ extern "C" int bshmem_moe_dispatch_local_noalloc(const void* x, const int* topk_
   a.expert_offsets = expert_offsets;
   a.src_offsets = nullptr;
   a.counts[0] = blk->counts;
-  a.flags[0] = blk->flags;
-  a.scratch = &blk->scratch;
   P.wait_limit_ns = 10000000000ull;
   return dispatch_local(P, stream);
 }

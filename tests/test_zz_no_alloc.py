@@ -117,6 +117,30 @@ def test_noalloc_dispatch_without_an_error_flag_keeps_its_error_bits_readable():
     _compare_on(_load(), 0, own_error_word=False)
 
 
+def test_noalloc_dispatch_clears_nothing_but_its_error_word():
+    """One stream operation of four bytes stands before the kernels: the count matrix is written whole by every call."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    lib = _load()
+    torch.cuda.set_device(0)
+    x = torch.randn(64, 256, device="cuda").to(torch.bfloat16)
+    idx = torch.randint(0, 8, (64, 2), device="cuda", dtype=torch.int32)
+    _noalloc(lib, x, idx, 8)  # looks the array up, outside the capture
+    recv, slot, offs = torch.empty(128, 256, dtype=torch.bfloat16, device="cuda"), torch.empty(64, 2, dtype=torch.int32, device="cuda"), torch.empty(9, dtype=torch.int32, device="cuda")
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        st = lib.bshmem_moe_dispatch_local_noalloc(x.data_ptr(), idx.data_ptr(), 64, 256, 2, 8, recv.data_ptr(), slot.data_ptr(), offs.data_ptr(), None,
+                                                   torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    cleared = 0
+    for node in driver.cuGraphGetNodes(raw, driver.cuGraphGetNodes(raw, 0)[2])[1]:
+        if driver.cuGraphNodeGetType(node)[1] == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_MEMSET:
+            err, p = driver.cuGraphMemsetNodeGetParams(node)
+            assert int(err) == 0
+            cleared += p.elementSize * p.width * max(1, p.height)
+    assert cleared == 4
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs a second GPU")
 def test_noalloc_dispatch_on_a_second_gpu_uses_that_gpus_array():
     """The array exists once per GPU and its address is looked up per GPU: the same two calls on device 1."""
