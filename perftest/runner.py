@@ -28,7 +28,8 @@ LISTS = {
     "coll": [("coll", ["--max-bytes", "128M", "--algos", "best"], None), ("tile", [], None)],
     "coll-all-algos": [("coll", ["--max-bytes", "32M", "--algos", "all", "--cold"], None)],
     "fused": [("fused", [], None), ("moe", [], None)],
-    "kernels": [("kernel_case", ["--kernel", k], (1,)) for k in ("gemm", "gemm_bench", "moe_dispatch", "moe_dispatch_fp8", "moe_combine", "allreduce")],
+    "kernels": [("kernel_case", ["--kernel", k], (1,)) for k in ("gemm", "gemm_bench", "gemm_decode", "moe_dispatch", "moe_dispatch_fp8", "moe_combine", "moe_dispatch_one_pe",
+                                                              "moe_dispatch_fp8_one_pe", "moe_combine_one_pe", "allreduce", "local_copy")],
 }
 LISTS["all"] = LISTS["p2p"] + LISTS["coll"] + LISTS["fused"] + LISTS["kernels"]
 
