@@ -246,26 +246,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
       if (!named_bar_and(1, EPI_THREADS, ok)) break;
       tc_fence_after_sync();
       const uint32_t t_row = tmem_base + ((uint32_t)(ew * 32) << 16) + (uint32_t)(acc * ACC_COLS);
-      auto release = [&] {  // hands the TMEM buffer back to the MMA warp
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) {
-          if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[acc]), 0));
-          else mbar_arrive(&acc_empty[acc]);
-        }
-      };
-      if (!staged_chunks(ti)) {  // one PE only: nothing is owed to a peer
-        release();
-        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
-        continue;
-      }
 #pragma unroll 1
       for (int c = 0; c < BN / EPI_COLS; ++c) {
         float f[EPI_COLS];
         tmem_ld_32x32(t_row + c * EPI_COLS, (uint32_t*)f);
         tmem_ld_32x32(t_row + c * EPI_COLS + 32, (uint32_t*)f + 32);
         tmem_ld_wait();
-        if (c == BN / EPI_COLS - 1) release();  // all of this accumulator is in registers
+        if (c == BN / EPI_COLS - 1) {
+          // All of this accumulator is in registers: hand the TMEM buffer back to the MMA warp.
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) {
+            if (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&acc_empty[acc]), 0));
+            else mbar_arrive(&acc_empty[acc]);
+          }
+        }
         if (p.act == BSHMEM_FUSED_ACT_GELU_TANH) {
           // tanh-approximated GELU on the fp32 accumulators, before the single rounding to bf16.
 #pragma unroll
@@ -307,7 +302,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
         }
         // Staging buffer (chunk_counter & 1) must have been drained by the TMA store issued two chunks ago.  Groups are counted,
         // not buffers: "all but the newest have been read" says that only because every staged chunk commits one group (an
-        // empty one where it leaves by other stores), whatever tile it belongs to.
+        // empty one where it is not stored, or by other stores), whatever tile it belongs to.  (Tiles without rows could skip
+        // all this, but the branch costs the others: 368.5 us in place of 365.6 at 8192 x 8192 x 3584.)
         uint8_t* buf = sE + (chunk_counter & 1) * EPI_BUF;
         if (issuer) bulk_wait_read<1>();
         named_bar_sync(1, EPI_THREADS);
@@ -334,7 +330,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) gemm_fused_kernel(const __grid_co
             const uint4 v = *(const uint4*)(buf + r * 128 + ((j ^ (r & 7)) << 4));
             multimem_st_v4(base + (size_t)r * p.N * 2 + j * 16, v);
           }
-        } else if (issuer) {
+        } else if (issuer && stored_chunks(ti)) {
           const int x = ti.n_tile * BN + c * EPI_COLS;
           if (sw) {
             tma_store_2d(&p.tmStage, buf, x, ti.m_tile * BM);
@@ -689,14 +685,14 @@ extern "C" int bshmem_fused_test_ag_units(int K, int grid, int* out) {
 // Test hook (host only): the tile width that plan_narrow chooses (0: the persistent kernel).
 extern "C" int bshmem_fused_test_narrow_plan(int tiles, int kblocks, double bytes, int sms) { return plan_narrow(tiles, kblocks, bytes, sms).n_tile; }
 
-// Test hook (host only): the chunks that the epilogue stages (and commits a group of stores for) at position `t` of the tile order of
-// one PE with `row_blocks` row blocks; -1 outside of it.
-extern "C" int bshmem_fused_test_staged_chunks(int M, int N, int row_blocks, int t) {
+// Test hook (host only): the chunks that the epilogue stores at position `t` of the tile order of one PE with `row_blocks` row blocks (it
+// stages all of them either way); -1 outside of it.
+extern "C" int bshmem_fused_test_stored_chunks(int M, int N, int row_blocks, int t) {
   if (M % BM || N % BN || row_blocks < M / BM || t < 0 || t >= row_blocks * (N / BN)) return -1;
   FusedParams p;
   memset(&p, 0, sizeof(p));
   p.mode = BSHMEM_FUSED_PLAIN; p.M = M; p.N = N; p.npes = 1; p.row_blocks = row_blocks;
-  return staged_chunks(tile_info(p, t));
+  return stored_chunks(tile_info(p, t));
 }
 
 // Test hook (host only): the tile that position `t` of the tile order names, for the checks of the order's

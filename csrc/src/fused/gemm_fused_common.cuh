@@ -77,9 +77,9 @@ __host__ __device__ __forceinline__ TileInfo tile_info(const FusedParams& p, int
   ti.valid_rows = ti.a_row < p.M ? BM : 0;
   return ti;
 }
-// Chunks of EPI_COLS columns that a tile sends through the epilogue's two staging buffers: none where there is no row to store.  (A chunk
-// that is staged but not stored would let the one after it overwrite a buffer that the copy engine still reads.)
-__host__ __device__ __forceinline__ int staged_chunks(const TileInfo& ti) { return ti.valid_rows ? BN / EPI_COLS : 0; }
+// Chunks of EPI_COLS columns, of those that a tile sends through the epilogue's two staging buffers, that are stored: none where there is
+// no row.
+__host__ __device__ __forceinline__ int stored_chunks(const TileInfo& ti) { return ti.valid_rows ? BN / EPI_COLS : 0; }
 __host__ __device__ __forceinline__ TileInfo tile_info_base(const FusedParams& p, int t) {
   const int tiles_n = p.N / BN;
   const int tmr = p.row_blocks ? p.row_blocks : (p.M / p.npes) / BM;

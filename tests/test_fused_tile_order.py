@@ -122,34 +122,37 @@ def test_narrow_plan_fits_one_wave():
                 assert width == next((w for w in (64, 128, 256) if tiles * (256 // w) <= sms), 0), (tiles, kblocks, sms)
 
 
-def _overwritten(staged_and_stored):
-    """Replays the epilogue's staging of one CTA: per tile (chunks staged, chunks stored).  Before a chunk writes buffer `counter & 1`, all
-    groups but the newest have been read.  Returns how often a buffer is written that a store may still be reading."""
-    bad, counter, pending = 0, 0, []          # pending: the buffer of every committed group, oldest first
-    for staged, stored in staged_and_stored:
-        for c in range(staged):
+def _overwritten(stored_per_tile, every_chunk_commits):
+    """Replays the epilogue's staging of one CTA: each tile stages four chunks, of which so many are stored.  Before a chunk writes buffer
+    `counter & 1`, all groups of stores but the newest have been read.  Returns how often a buffer is written that a store may
+    still be reading."""
+    bad, counter, pending = 0, 0, []          # pending: the buffer that every committed group reads (None: empty group), oldest first
+    for stored in stored_per_tile:
+        for c in range(4):
             pending = pending[-1:]
             bad += (counter & 1) in pending
             if c < stored:
                 pending.append(counter & 1)
+            elif every_chunk_commits:
+                pending.append(None)
             counter += 1
     return bad
 
 
 @pytest.mark.parametrize("M,N", [(4224, 8192), (8320, 8192), (4480, 3584), (1152, 8448), (2176, 2304), (8192, 8192)])
 def test_no_staging_buffer_is_written_while_a_store_reads_it(M, N):
-    """Row blocks rounded up to pairs, tiles dealt to 148 CTAs as the persistent kernel deals them: the added block stages nothing.
-    Were its chunks staged and not stored, buffers would be overwritten."""
+    """Row blocks rounded up to pairs, tiles dealt to 148 CTAs as the persistent kernel deals them.  The added block is staged and not
+    stored; its chunks commit a group all the same.  Did only stored chunks commit, buffers would be overwritten."""
     lib = _lib()
-    lib.bshmem_fused_test_staged_chunks.argtypes = [C.c_int] * 4
+    lib.bshmem_fused_test_stored_chunks.argtypes = [C.c_int] * 4
     blocks = M // BM + (M // BM) % 2
     total, odd = blocks * (N // BN), (M // BM) % 2
-    chunks = [lib.bshmem_fused_test_staged_chunks(M, N, blocks, t) for t in range(total)]
-    assert lib.bshmem_fused_test_staged_chunks(M, N, blocks, total) == -1
+    chunks = [lib.bshmem_fused_test_stored_chunks(M, N, blocks, t) for t in range(total)]
+    assert lib.bshmem_fused_test_stored_chunks(M, N, blocks, total) == -1
     assert chunks.count(4) == M // BM * (N // BN) and chunks.count(0) == odd * (N // BN) and len(chunks) == total
     per_cta = [chunks[first::148] for first in range(148)]
-    assert sum(_overwritten([(c, c) for c in tiles]) for tiles in per_cta) == 0
-    planted = sum(_overwritten([(4, c) for c in tiles]) for tiles in per_cta)
+    assert sum(_overwritten(tiles, True) for tiles in per_cta) == 0
+    planted = sum(_overwritten(tiles, False) for tiles in per_cta)
     assert (planted > 0) == any(a == 4 and b == 0 for tiles in per_cta for a, b in zip(tiles, tiles[1:]))
 
 
