@@ -1,12 +1,16 @@
 // C interface of the expert-parallel dispatch / combine kernels (libbshmem_fused.so).
 //
 // dispatch: every PE holds T tokens of H bf16 values and, per token, K expert ids out of E
-// (expert e lives on PE e / (E/npes)).  One cooperative kernel counts, exchanges the counts with
-// all PEs, derives where each (token, expert) pair lands and pushes the rows straight into the
-// receive buffer of the owning PE, grouped by expert, then by source PE.  The rows travel as bf16
-// or as fp8 e4m3 with one fp32 scale per 128 values (quantised on the fly).  One PE (without dup_src) runs one or two plain kernels instead.
+// (expert e lives on PE e / (E/npes)).  The rows of all (token, expert) pairs end up in the receive
+// buffer of the expert's PE, grouped by expert, then by source PE.  They travel as bf16 or as fp8
+// e4m3 with one fp32 scale per 128 values (quantised on the fly).
+//   several PEs, or dup_src given: one cooperative kernel counts, exchanges the counts with all PEs,
+//     derives where each pair lands and pushes the rows straight into the receive buffers
+//   one PE: no barrier and no cooperative launch; one kernel that counts and places by itself for up
+//     to 2048 pairs, above that a routing kernel and one that only moves rows.  `flags` and `scratch`
+//     are not used (they must be given all the same)
 // combine: the inverse; every PE pulls, for each of its tokens, the K expert outputs from the PEs
-// that own them and writes their weighted sum.
+// that own them and writes their weighted sum.  (One PE: a plain launch without barriers.)
 // The library allocates nothing: receive buffers, the count matrix and the flags are symmetric
 // buffers supplied by the caller (the peers' mapped addresses of the same objects), the small
 // scratch block is local device memory.
@@ -54,7 +58,7 @@ typedef struct {
   /* Optional: [cap_rows] int32 on every PE (symmetric).  When set, a token that goes to several experts of one PE
    * crosses NVLink once: its row is written to the first of its rows on that PE, the other rows receive only the
    * number of that first row here, and the receiving PE copies the row locally before the kernel ends.  Null on every
-   * entry = every (token, expert) pair is sent (the only form with one PE). */
+   * entry = every (token, expert) pair is sent. */
   int* dup_src[BSHMEM_MOE_MAX_PES];
 } bshmem_moe_dispatch_args_t;
 

@@ -149,8 +149,11 @@ static int ctas_for(size_t bytes, size_t threshold) {
 // Every data collective of a team of one is a copy of its source, unless the caller names an algorithm (that runs the kernel for
 // several members as ever, on its few CTAs).  Nothing has to be met or flagged, so the launch is not
 // tied to the rows of barrier flags (32 CTAs at most) and fills the GPU: bound by HBM.  256 threads keep four 16-byte
-// loads each in flight, eight CTAs fit an SM, so 128 KB per SM are on their way; a CTA takes 16 KB per round.
-// 256 MB read and 256 MB written: 213 us with 32 CTAs of 512 threads, 89 us here (6.06 TB/s).
+// loads each in flight; 48 registers let five CTAs fit an SM, so 80 KB per SM are on their way, and a CTA takes 16 KB per round.
+// The grid is eight CTAs per SM: three start as others end, which large copies like better than a grid of what fits.  16 / 64 / 256 /
+// 512 MB read and written, us: eight per SM 5.5 / 16.6 / 85.9 / 172.7 (6.2 TB/s), five per SM 5.2 / 17.0 / 89.5 / 180.8, eight of 32
+// registers (all resident) 5.2 / 17.8 / 89.6 / 180.3; 256 MB with 32 CTAs of 512 threads 213.
+// A copy that is to leave SMs to other work is given fewer CTAs by NVSHMEM_MAX_CTAS, or by naming an algorithm.
 static constexpr int kCopyThreads = 256, kCopyUnroll = 4, kCopyCtasPerSm = 8;
 
 template <class V>

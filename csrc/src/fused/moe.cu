@@ -461,6 +461,11 @@ __global__ void __launch_bounds__(THREADS, (KT <= 8 ? 3 : 2) + (LOCAL ? 1 : 0)) 
 //    L2) and finds the place of its own token's rows by counting the equal ids before them;
 //  * more: a routing kernel (one cluster of eight CTAs, counts met through distributed shared memory) writes the slot map and
 //    the offsets, then a kernel that only moves rows.
+// The line lies at 2048 pairs because every item of the one kernel scans the pairs before it.  One kernel / two, us: 7168 values, top-8 of
+// 256, bf16: 1024 pairs 7.0 / 8.1, 2048 9.0 / 11.0, 4096 14.5 / 15.7, 8192 31.4 / 25.2; fp8: 2048 7.9 / 9.5, 4096 12.2 / 11.3; 1024 values:
+// 2048 6.2 / 7.4, 4096 8.3 / 7.6; 512 values, top-16 of 64: 2048 5.5 / 7.2, 3072 7.7 / 7.0.
+// Routing CTAs: eight is the largest cluster that needs no opt-in; 8192 tokens of 128 values, fp8, top-8: 11.7 us with eight, 16.4 with
+// four, 26.0 with two.
 // Device time, 64 tokens x 7168, top-8 of 256: 16.5 us before, 7 us now; 4096 tokens: bf16 112 us -> 6.3 (routing) + 91
 // (529 MB, 5.8 TB/s), fp8 79.6 us -> 6.5 + 51.5 (5.8 TB/s), bound by HBM writes.  The row kernel is launched early and loads
 // token rows while the routing runs (2.5 us less).
@@ -686,6 +691,8 @@ static_assert(BSHMEM_MOE_MAX_EXPERTS <= ROUTE_THREADS, "one thread per expert");
 // Rows of a large batch, bf16: every warp runs a ring of PUSH_DEPTH shared-memory buffers that the bulk-copy engine fills
 // from a piece of a token's row and empties into the K receive rows, lane k issuing the copy to row k: no register or
 // load / store unit touches the data, and one load feeds K stores.
+// 4096 tokens of 7168 / 512 values, top-8, us with the routing: 4 warps x 4 buffers of 4 KB 96.5 / 12.0, of 2 KB 97.1 / 11.8, of 8 KB
+// 96.4 / 12.7, 8 warps of 2 KB 97.3 / 12.7.
 constexpr int PUSH_WARPS = 4, PUSH_DEPTH = 4, PUSH_BYTES = 4096;
 constexpr int PUSH_SMEM = PUSH_WARPS * PUSH_DEPTH * PUSH_BYTES;
 
