@@ -13,13 +13,14 @@
 //             memory and stored as whole 128- or 256-byte pieces of output rows
 // The ring's stages are as large as the largest chunk of the call needs: small groups leave room for more stages, which is
 // what keeps enough weight bytes in flight when the weights' HBM traffic is the bound.
-// Large groups are bound by the tensor cores at the clock that the power limit leaves (94 % of cycles active at 1.2 GHz), small
-// ones by HBM.  Rows as the first operand in blocks of 128 (before) / weights first in CTA pairs (now), us, sizes within
+// Large groups are bound by the clock that the power limit leaves (K 7168, 1024 rows: 1.04 GHz in a loop of seconds, MMAs in 0.885 of the
+// cycles), small ones by HBM.  Rows as the first operand in blocks of 128 (before) / weights first in CTA pairs (now), us, sizes within
 // 10 % of the mean:
 //   32 groups, N 4096, K 7168, gated   16 rows 328 / 272 (1.88 GB of weights: 6.9 TB/s)   256 631 / 505   1024 1741 / 1695
 //   32 groups, N 7168, K 2048          16 rows 156 / 146 (0.94 GB)                        256 295 / 251   1024 1015 / 782
 //   32 groups, N 2048, K 512           16 rows 12.4 / 12.3                                256 32.5 / 27.6  1024 88.9 / 69.9
 //   256 groups, N 512, K 512           16 rows 40.6 / 30.0                                256 68.5 / 54.3
+// These are short runs; a whole layer of 4096 tokens (1024 rows a group) gains nothing in a loop of seconds, at 512 to 2048 tokens 4 to 18 %.
 // One epilogue warpgroup instead of two: 120 us in place of 69.9, and 27 % more than now at 16 x 1024 x 1024, 1024 rows.
 #pragma once
 #include "gemm_fused_common.cuh"
